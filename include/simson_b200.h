@@ -323,17 +323,17 @@ int sgpu_stream(sgpu_ctx* ctx, void** stream);
 int sgpu_cfl_partial(sgpu_ctx* ctx, double* cflp, int* pending);
 int sgpu_cfl_set_global(sgpu_ctx* ctx, double cflp);
 
-/* Step 3's pencil kernel: warp = 1 solves each (kx, kz) pencil with one warp
- * (every column of the pencil in registers across the warp: the tau solves
- * by the partition method with a parallel cyclic reduction over the lanes,
- * the Chebyshev derivatives as warp scans), warp = 0 with one thread per
- * pencil sweeping its columns through memory in the reference's elimination
- * order (bla/trid.f:120-200), warp = 2 chooses: the warp kernel up to 8192
- * pencils (nz nx/2; grids such as the LES grid 64x97x64, where one thread
- * per pencil leaves the GPU idle), the thread kernel above (the default,
- * also set at sgpu_init; SIMSON_PENCIL_WARP=0/1 in the environment forces
- * one for new contexts).  Both solve the same tau systems, to round-off.
- * SGPU_E_PARAM for warp = 1 when ny > 256. */
+/* Step 3's pencil kernel: warp = 1 solves each (kx, kz) pencil with a group of
+ * threads (each a chunk of its Chebyshev rows in registers: the tau solves as
+ * chunk recurrences joined by a walk over the chunks, the Chebyshev
+ * derivatives likewise; under SGPU_MIXED a warp with a cyclic reduction
+ * over its lanes), warp = 0 with one thread per pencil sweeping its
+ * columns through memory in the reference's elimination order
+ * (bla/trid.f:120-200), warp = 2 chooses: the group, except under SGPU_MIXED
+ * above 8192 pencils (nz nx/2) (the default, also set at sgpu_init;
+ * SIMSON_PENCIL_WARP=0/1 in the environment forces one for new contexts).
+ * All solve the same tau systems, to round-off.  SGPU_E_PARAM for warp = 1
+ * when ny > 256. */
 int sgpu_set_pencil_kernel(sgpu_ctx* ctx, int warp);
 
 /* Failure detection of the tensor-core kernels (the mixed path's Chebyshev

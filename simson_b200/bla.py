@@ -288,8 +288,8 @@ class Channel:
         return n.value
 
     def set_pencil_kernel(self, warp=True):
-        """Step 3 with one warp per pencil (True), one thread per pencil
-        (False) or the automatic choice by grid size ("auto");
+        """Step 3 with a group of threads per pencil (True), one thread per
+        pencil (False) or the automatic choice by grid size ("auto");
         sgpu_set_pencil_kernel."""
         self._check(self.lib.sgpu_set_pencil_kernel(self._ctx, 2 if warp == "auto" else int(bool(warp))),
                     "set_pencil_kernel")

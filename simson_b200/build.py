@@ -13,9 +13,10 @@ ROOT = os.path.dirname(HERE)
 LIB_DIR = os.path.join(HERE, "_lib")
 LIB = os.path.join(LIB_DIR, "libsimson_b200.so")
 SOURCES = [os.path.join(HERE, "csrc", "simson.cu"), os.path.join(HERE, "csrc", "noalloc.cu"),
-           os.path.join(HERE, "csrc", "mixed.cu")]
-# units built with fused multiply-add contraction (the mixed-precision path)
-FMAD_SOURCES = {os.path.join(HERE, "csrc", "mixed.cu")}
+           os.path.join(HERE, "csrc", "mixed.cu"), os.path.join(HERE, "csrc", "pencil_chunk.cu")]
+# units built with fused multiply-add contraction (the mixed-precision path,
+# the chunked pencil kernel)
+FMAD_SOURCES = {os.path.join(HERE, "csrc", "mixed.cu"), os.path.join(HERE, "csrc", "pencil_chunk.cu")}
 DEPS = [os.path.join(HERE, "csrc", f) for f in os.listdir(os.path.join(HERE, "csrc"))] + [
     os.path.join(ROOT, "include", "simson_b200.h")]
 ARCH = "-gencode=arch=compute_100a,code=sm_100a"

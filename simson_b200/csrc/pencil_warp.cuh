@@ -1,4 +1,5 @@
-// Step 3 with one warp per (kx, kz) pencil: the same algebra as k_pencil
+// Step 3 of the mixed path with one warp per (kx, kz) pencil (the FP64 path:
+// pencil_chunk.cuh): the same algebra as k_pencil
 // (bla/linearbl.f:257-1860 for the channel, ibc = 0, tau method), with every
 // column of the pencil held in registers across the warp instead of being
 // swept serially by one thread through memory.

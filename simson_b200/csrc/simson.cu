@@ -29,6 +29,7 @@
 #include "mixed.h"
 #include "step2_launch.cuh"
 #include "cheb_tc.cuh"
+#include "pencil_chunk.h"
 #include "pencil_warp.cuh"
 
 using namespace sb;
@@ -91,6 +92,14 @@ struct sgpu_ctx {
   double* hom_cf = nullptr;  // coefficient columns [3][4][nyp][NP] (k_pencil_hom)
   double hom_key[4] = {0.0, 0.0, 0.0, 0.0};
   int hom_next = 0;
+  // chunked pencil kernel (pencil_chunk.cuh): eliminated tau coefficients of
+  // (D^2 - lam) per RK stage and of (D^2 - k^2), [nyp][(nz/2 + 1) nx/2] each,
+  // keyed like the homogeneous solutions, and the row factors
+  double* tau_l = nullptr;
+  double* tau_v = nullptr;
+  double2* tau_rows = nullptr;
+  double tau_key[4] = {0.0, 0.0, 0.0, 0.0};
+  int tau_next = 0;
   double* mscr = nullptr;    // mean-flow scratch
   double* meanp = nullptr;   // [4][nyp] U, W, Omega_x, Omega_z for the mixed step 2
   double* ampd = nullptr;    // [20][nyp] plane statistics
@@ -176,9 +185,9 @@ struct sgpu_ctx {
   static constexpr int kbf = MIXED_KB, rbf = MIXED_RB, pbf = 8;  // FP32 tiles (mixed.h)
   // optional per-kernel timing (sgpu_profile): event pairs around each launch
   bool prof = false;
-  // step 3 with one warp per pencil (pencil_warp.cuh) instead of one thread
-  // per pencil (k_pencil); SIMSON_PENCIL_WARP=0/1 overrides the default
-  bool pencil_warp = false;
+  // step 3 with a group of threads per pencil (pencil_chunk.cuh, pencil_warp.cuh)
+  // instead of one thread per pencil (k_pencil); SIMSON_PENCIL_WARP=0/1 overrides the default
+  bool pencil_group = false;
   // bounded waits of the tensor-core kernels (sgpu_set_wait_limit)
   int wait_limit = 0;
   int test_timeout = 0;
@@ -195,8 +204,26 @@ struct sgpu_ctx {
   int pnext = 0;
 };
 
-// the warp-per-pencil step 3 up to this many pencils (auto selection)
-constexpr int kPencilWarpMaxPencils = 8192;
+// Whether a group of threads can solve a pencil of this context.  FP64: the
+// chunked kernel.  Mixed: one warp per pencil; the chunked kernel would serve
+// its FP32 storage as well (64x97x64 0.021 against 0.062 ms), but joins its
+// sums in another order, and the mixed path's forcing, rounded to FP32, turns
+// a last-bit difference into its whole rounding noise (4e-6 of p_v, single
+// values up to 7e-4 of its rms), beyond what a change of kernel may show.
+static bool pencil_chunked(const sgpu_ctx* c) { return !c->mixed && pencil_chunk_fits(c->g.nyp); }
+static bool pencil_group_fits(const sgpu_ctx* c) {
+  return c->mixed ? pencil_warp_rows(c->g.nyp) > 0 : pencil_chunk_fits(c->g.nyp) != 0;
+}
+// The automatic choice of step 3's pencil kernel.  FP64: the chunked kernel
+// (against one thread per pencil: 48x65x48 0.012 / 0.24 ms, 192x129x160 0.18 /
+// 0.59, 384x193x384 1.25 / 1.81).  Mixed: a warp per pencil up to 8192 pencils
+// (0.062 against 0.29 ms at 64x97x64, 2 048 pencils; 0.28 against 0.58 at
+// 96x129x96, 4 608), one thread per pencil above (0.43 against 0.85 at
+// 192x129x160, 15 360; 1.0 against 5.2 at 384x193x384, 73 728, where it
+// streams near the DRAM bandwidth).
+static bool pencil_group_auto(const sgpu_ctx* c) {
+  return pencil_group_fits(c) && (!c->mixed || c->g.NP <= 8192);
+}
 
 enum KernelId { K_ZINV = 0, K_XPASS, K_ZFWD, K_CHEB_FWD, K_PENCIL, K_MEAN, K_CHEB_INV, K_OTHER, K_COUNT };
 
@@ -346,6 +373,33 @@ extern "C" const char* sgpu_error_string(int code) {
 
 static size_t smem_fft(int n, int cols, size_t elem) { return 2 * (size_t)n * cols * elem; }
 
+// The buffers of the selected pencil kernel (both keep theirs once made): the
+// homogeneous solutions and coefficient columns of the thread-per-pencil
+// kernel, or the tau coefficients of the chunked one, whose (D^2 - k^2) part
+// does not depend on the time step and is computed here.
+static int pencil_bufs(sgpu_ctx* c) {
+  const Dims& g = c->g;
+  const size_t fld = (size_t)g.nyp * g.NP, nst = (size_t)c->prm.nst;
+  if (!c->pencil_group) {
+    if ((!c->hom_vh && cudaMalloc(&c->hom_vh, nst * fld * sizeof(double)) != cudaSuccess) ||
+        (!c->hom_s && cudaMalloc(&c->hom_s, nst * 2 * (size_t)g.NP * sizeof(double)) != cudaSuccess) ||
+        (!c->hom_cf && cudaMalloc(&c->hom_cf, nst * 4 * fld * sizeof(double)) != cudaSuccess))
+      return SGPU_E_CUDA;
+    return SGPU_OK;
+  }
+  if (!pencil_chunked(c) || c->tau_rows) return SGPU_OK;
+  const size_t col = (size_t)g.nyp * (g.nz / 2 + 1) * g.nx2;
+  const std::vector<double2> rows = pencil_chunk_table(g.nyp);
+  if ((!c->tau_l && cudaMalloc(&c->tau_l, nst * col * sizeof(double)) != cudaSuccess) ||
+      (!c->tau_v && cudaMalloc(&c->tau_v, col * sizeof(double)) != cudaSuccess) ||
+      cudaMalloc(&c->tau_rows, rows.size() * sizeof(double2)) != cudaSuccess)
+    return SGPU_E_CUDA;
+  CK(cudaMemcpyAsync(c->tau_rows, rows.data(), rows.size() * sizeof(double2), cudaMemcpyHostToDevice, c->stream));
+  pencil_tau_coef(c->stream, c->tau_v, g, c->alfa, c->beta, 0.0);
+  CK(cudaStreamSynchronize(c->stream));
+  return SGPU_OK;
+}
+
 extern "C" int sgpu_init(const sgpu_params* prm, sgpu_ctx** out) {
   if (!prm || !out) return SGPU_E_PARAM;
   *out = nullptr;
@@ -395,9 +449,6 @@ extern "C" int sgpu_init(const sgpu_params* prm, sgpu_ctx** out) {
       cudaMalloc(&c->cz, (size_t)c->ncz * fld * sizeof(double2)) != cudaSuccess ||
       cudaMalloc(&c->rz, (size_t)c->nrz * fld * sizeof(double)) != cudaSuccess ||
       cudaMalloc(&c->mscr, 16 * (size_t)g.nyp * sizeof(double)) != cudaSuccess ||
-      cudaMalloc(&c->hom_vh, (size_t)P.nst * fld * sizeof(double)) != cudaSuccess ||
-      cudaMalloc(&c->hom_s, (size_t)P.nst * 2 * (size_t)g.NP * sizeof(double)) != cudaSuccess ||
-      cudaMalloc(&c->hom_cf, (size_t)P.nst * 4 * fld * sizeof(double)) != cudaSuccess ||
       cudaMalloc(&c->stage, 2 * 7 * fld * sizeof(double)) != cudaSuccess ||
       cudaMalloc(&c->ampd, 20 * (size_t)g.nyp * sizeof(double)) != cudaSuccess)
     return fail(SGPU_E_CUDA);
@@ -466,14 +517,10 @@ extern "C" int sgpu_init(const sgpu_params* prm, sgpu_ctx** out) {
   // SIMSON_GRAPHS=0: launch every kernel directly (no CUDA-graph replay)
   const char* ge = getenv("SIMSON_GRAPHS");
   c->graphs = !(ge && ge[0] == '0');
-  // step 3's pencil kernel: one warp per pencil on grids with few pencils
-  // (its parallelism is per pencil: 0.11 against 0.42 ms at 64x97x64, 2 048
-  // pencils; 0.28 against 0.58 ms at 96x129x96, 4 608), one thread per
-  // pencil on large grids (0.58 against 0.85 ms at 192x129x160, 15 360; 1.3
-  // against 5.2 ms at 384x193x384, 73 728, where the thread kernel streams
-  // near the DRAM bandwidth); SIMSON_PENCIL_WARP=0/1 forces one of them
+  // SIMSON_PENCIL_WARP=0/1 forces one of step 3's pencil kernels
   const char* pw = getenv("SIMSON_PENCIL_WARP");
-  c->pencil_warp = pencil_warp_rows(g.nyp) > 0 && (pw ? pw[0] == '1' : g.NP <= kPencilWarpMaxPencils);
+  c->pencil_group = pw ? (pw[0] == '1' && pencil_group_fits(c)) : pencil_group_auto(c);
+  if ((rc = pencil_bufs(c))) return fail(rc);
   if (cudaDeviceSynchronize() != cudaSuccess) return fail(SGPU_E_CUDA);
   *out = c;
   return SGPU_OK;
@@ -488,7 +535,7 @@ extern "C" int sgpu_finalize(sgpu_ctx* c) {
                   c->sgs_delta2, c->sgs_twz.d, c->sgs_twz.f, c->sgs_twx.d, c->sgs_twx.f, c->xys, c->xys_spec,
                   c->xys_part, c->xys_u, c->box_out, c->press, c->press_wd, c->xys_twz.d, c->xys_twz.f, c->xys_twx.d, c->xys_twx.f, c->mlp_image, c->mlp_tau,
                   c->mlp_err, c->sgs_flags, c->sgs_bsums, c->chb_fwd, c->chb_inv, c->chb_err, c->puw, c->scal, c->cfl_bits, c->alfa, c->beta, c->dyi, c->zb, c->xb, c->cz, c->rz,
-                  c->mscr, c->hom_vh, c->hom_s, c->hom_cf, c->stage, c->twz.d, c->twz.f, c->twx.d, c->twx.f, c->twy.d, c->twy.f,
+                  c->mscr, c->hom_vh, c->hom_s, c->hom_cf, c->tau_l, c->tau_v, c->tau_rows, c->stage, c->twz.d, c->twz.f, c->twx.d, c->twx.f, c->twy.d, c->twy.f,
                   c->fr_lam, c->fr_base, c->les_lpf2, c->les_filt2, c->les_gu2, c->hpf_s2};
   for (void* p : ptrs)
     if (p) cudaFree(p);
@@ -1027,17 +1074,18 @@ static int enqueue_linear(sgpu_ctx* c) {
   M.cflux = P.cflux;
   // the mean flow belongs to the context that owns pencil 0 (kz = 0)
   const bool own_mean = g.p0 == 0;
-  // the warp kernels of step 3 come with the warp mean-flow solve
+  const bool chunked = c->pencil_group && pencil_chunked(c);
   auto mean = [&](cudaStream_t st) {
-    if (c->pencil_warp && (c->mixed ? launch_mean_warp<float2>(st, M, g, P.re, rk)
-                                    : launch_mean_warp<double2>(st, M, g, P.re, rk)))
-      return;
+    c->launches++;
+    if (c->pencil_group && launch_mean_warp<float2>(st, M, g, P.re, rk)) return;
     if (c->mixed)
       mixed_mean(st, M, g, P.re, rk);
     else
       k_mean<double2><<<1, 32, 0, st>>>(M, g, P.re, rk);
   };
-  if (!own_mean) {
+  // (the chunked pencil kernel solves it in a CTA of its own)
+  const bool side = own_mean && !chunked && !c->prof;
+  if (!own_mean || chunked) {
   } else if (c->prof) {
     prof_mark(c, K_MEAN);
     mean(c->stream);
@@ -1047,13 +1095,29 @@ static int enqueue_linear(sgpu_ctx* c) {
     mean(c->side);
     cudaEventRecord(c->join, c->side);
   }
-  if (c->pencil_warp) {
-    // one warp per pencil: the homogeneous solutions are columns of its own
-    // solves, no per-stage cache
+  if (c->pencil_group && !chunked) {
+    // mixed: one warp per pencil, no per-stage cache
     prof_mark(c, K_PENCIL);
-    const bool ok = c->mixed ? mixed_pencil_warp(c->stream, B, g, c->alfa, c->beta, P.re, rk)
-                             : launch_pencil_warp<double2, double>(c->stream, B, g, c->alfa, c->beta, P.re, rk);
-    if (!ok) return SGPU_E_PARAM;
+    if (!mixed_pencil_warp(c->stream, B, g, c->alfa, c->beta, P.re, rk)) return SGPU_E_PARAM;
+  } else if (c->pencil_group) {
+    // this stage's tau coefficients, computed on its first use
+    const double anbn = rk.an + rk.bn;
+    const size_t col = (size_t)g.nyp * (g.nz / 2 + 1) * g.nx2;
+    int ts = -1;
+    for (int s = 0; s < c->prm.nst; ++s)
+      if (c->tau_key[s] == anbn) ts = s;
+    if (ts < 0) {
+      ts = c->tau_next;
+      c->tau_next = (c->tau_next + 1) % c->prm.nst;
+      c->tau_key[ts] = anbn;
+      prof_mark(c, K_OTHER);
+      pencil_tau_coef(c->stream, c->tau_l + ts * col, g, c->alfa, c->beta, 2.0 * P.re / anbn);
+      c->launches++;
+    }
+    prof_mark(c, K_PENCIL);
+    if (!pencil_chunk(c->stream, B, g, c->alfa, c->beta, P.re, rk, c->tau_l + ts * col, c->tau_v,
+                      c->tau_rows, own_mean ? &M : nullptr))
+      return SGPU_E_PARAM;
   } else {
   // this stage's homogeneous solutions, computed on its first use (a key of
   // 0 is never a valid a_n + b_n: dt > 0)
@@ -1086,14 +1150,14 @@ static int enqueue_linear(sgpu_ctx* c) {
     k_pencil<double2, double, double><<<(g.p1 - g.p0 + 127) / 128, 128, 0, c->stream>>>(B, g, c->alfa, c->beta, P.re, rk,
                                                                                  vhc, hsc, cfc);
   }
-  if (!c->prof && own_mean) cudaStreamWaitEvent(c->stream, c->join, 0);
+  if (side) cudaStreamWaitEvent(c->stream, c->join, 0);
   // u, v, w, omega_x, omega_z back to physical y (slots 0-4), oddball plane untouched
   prof_mark(c, K_CHEB_INV);
   cheb_to_phys(c, B.OU, 0, 5, 1, /*fp32_input=*/c->mixed);
   // ADM-RT and HPF: high-pass filtered new velocities (bla/linearbl.f:1871-2060)
   if (c->iles == 1 || c->iles == 3) les_filter_velocity(c, 1);
   prof_mark(c, K_OTHER);
-  c->launches += 2;
+  c->launches++;  // the pencil kernel
   it_advance(c);
   return cuda_fail(cudaGetLastError(), "linear launch");
 }
@@ -1213,18 +1277,18 @@ extern "C" int sgpu_cfl_set_global(sgpu_ctx* c, double cflp) {
 // bit 9 the fringe.
 // 0xffffffff: the step cannot be replayed (not at a step boundary, its time
 // step changes at its end, or a stage's homogeneous solutions not yet
-// cached: that substep launches k_pencil_hom).
+// or tau coefficients not yet cached: that substep launches their kernel).
 static unsigned step_pattern(const sgpu_ctx* c) {
   const int nst = c->prm.nst;
   if ((c->it - 1) % nst != 0 || c->dt_next != c->dtn) return 0xffffffffu;
-  unsigned key = ((unsigned)c->iles << 4) | ((c->pencil_warp ? 1u : 0u) << 8) | ((c->fringe ? 1u : 0u) << 9);
+  unsigned key = ((unsigned)c->iles << 4) | ((c->pencil_group ? 1u : 0u) << 8) | ((c->fringe ? 1u : 0u) << 9);
   double anp1 = c->anp1, bnp1 = c->bnp1;
   for (int s = 0; s < nst; ++s) {
     const int it = c->it + s;
     if (c->prm.icfl > 0 && (it - 1) % c->prm.icfl == 0) key |= 1u << s;
     const double anbn = anp1 + bnp1;  // a_n + b_n of this substep's linear step
-    bool cached = c->pencil_warp;  // the warp kernel keeps no per-stage cache
-    for (int h = 0; h < nst; ++h) cached = cached || c->hom_key[h] == anbn;
+    bool cached = c->pencil_group && !pencil_chunked(c);  // the warp kernel keeps no per-stage cache
+    for (int h = 0; h < nst; ++h) cached = cached || (c->pencil_group ? c->tau_key[h] : c->hom_key[h]) == anbn;
     if (!cached) return 0xffffffffu;
     anp1 = c->dtn * ANRK[nst - 3][it % nst];
     bnp1 = c->dtn * BNRK[nst - 3][it % nst];
@@ -1474,10 +1538,9 @@ extern "C" int sgpu_get_scalars(sgpu_ctx* c, double* out, int n) {
 extern "C" int sgpu_set_pencil_kernel(sgpu_ctx* c, int warp) {
   if (c) c->step_valid = false;  // the captured step launches the other kernel
   if (!c || warp < 0 || warp > 2) return SGPU_E_PARAM;
-  const bool fits = pencil_warp_rows(c->g.nyp) > 0;
-  if (warp == 1 && !fits) return SGPU_E_PARAM;
-  c->pencil_warp = warp == 2 ? (fits && c->g.NP <= kPencilWarpMaxPencils) : warp == 1;
-  return SGPU_OK;
+  if (warp == 1 && c->g.nyp > 256) return SGPU_E_PARAM;
+  c->pencil_group = warp == 2 ? pencil_group_auto(c) : (warp == 1 && pencil_group_fits(c));
+  return pencil_bufs(c);
 }
 
 extern "C" int sgpu_set_wait_limit(sgpu_ctx* c, int limit, int test_timeout) {
