@@ -12,11 +12,11 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 LIB_DIR = os.path.join(HERE, "_lib")
 LIB = os.path.join(LIB_DIR, "libsimson_b200.so")
-SOURCES = [os.path.join(HERE, "csrc", "simson.cu"), os.path.join(HERE, "csrc", "noalloc.cu"),
-           os.path.join(HERE, "csrc", "mixed.cu"), os.path.join(HERE, "csrc", "pencil_chunk.cu")]
-# units built with fused multiply-add contraction (the mixed-precision path,
-# the chunked pencil kernel)
-FMAD_SOURCES = {os.path.join(HERE, "csrc", "mixed.cu"), os.path.join(HERE, "csrc", "pencil_chunk.cu")}
+UNITS = ["simson", "noalloc", "mixed", "pencil_chunk", "cheb_f64", "step2_f64"] + ["step2_f64_" + u for u in "abcd"]
+SOURCES = [os.path.join(HERE, "csrc", u + ".cu") for u in UNITS]
+# units built without fused multiply-add contraction: the host unit with the
+# kernels that keep the reference's rounding, and the allocation-free step 2
+NO_FMAD_SOURCES = {os.path.join(HERE, "csrc", u + ".cu") for u in ("simson", "noalloc")}
 DEPS = [os.path.join(HERE, "csrc", f) for f in os.listdir(os.path.join(HERE, "csrc"))] + [
     os.path.join(ROOT, "include", "simson_b200.h")]
 ARCH = "-gencode=arch=compute_100a,code=sm_100a"
@@ -40,17 +40,17 @@ def build(force: bool = False, verbose: bool = False) -> str:
     if not force and not needs_build():
         return LIB
     os.makedirs(LIB_DIR, exist_ok=True)
-    # The FP64 path is built without FMA contraction: the reference's
-    # arithmetic (gfortran/gcc for x86-64) rounds every product, and the stiff
-    # tau solves (lambda ~ 1e6) amplify the difference between fused and
-    # separate rounding to ~1e-12.  Set SIMSON_FMAD=1 to allow contraction.
-    # The mixed-precision unit is built with contraction (it is checked
-    # against the FP64 path at 1e-5, not bit for bit).
+    # The thread-per-pencil FP64 path is built without FMA contraction: the
+    # reference's arithmetic (gfortran/gcc for x86-64) rounds every product, and
+    # the stiff tau solves (lambda ~ 1e6) amplify the difference between fused
+    # and separate rounding to ~1e-12.  Set SIMSON_FMAD=1 to allow contraction.
+    # The other units (the mixed path, the chunked pencil kernel, the two-pass
+    # FP64 transforms) order their sums their own way and are built with it.
     fmad_all = os.environ.get("SIMSON_FMAD") == "1"
     objs = []
     procs = []
     for src in SOURCES:
-        fmad = "true" if (fmad_all or src in FMAD_SOURCES) else "false"
+        fmad = "true" if (fmad_all or src not in NO_FMAD_SOURCES) else "false"
         obj = os.path.join(LIB_DIR, os.path.splitext(os.path.basename(src))[0] + ".o")
         cmd = [nvcc(), ARCH, "-O3", "-lineinfo", "-std=c++17", f"-fmad={fmad}", "-Xcompiler", "-fPIC",
                "--expt-relaxed-constexpr", "-c", src, "-o", obj]

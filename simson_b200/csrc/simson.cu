@@ -28,6 +28,7 @@
 #include <nvtx3/nvToolsExt.h>
 #include "mixed.h"
 #include "step2_launch.cuh"
+#include "step2_f64.h"
 #include "cheb_tc.cuh"
 #include "pencil_chunk.h"
 #include "pencil_warp.cuh"
@@ -613,19 +614,26 @@ static void launch_cheb_t(sgpu_ctx* c, const typename C2<SI>::type* in, size_t i
                           size_t out_fs, int nfields, int inverse, double scale, int skip_oddball,
                           const typename C2<T>::type* tw) {
   const Dims& g = c->g;
+  if constexpr (sizeof(T) == 8) {
+    if (f2_cheb(c->stream, in, in_fs, out, out_fs, g, nfields, inverse, scale, tw, skip_oddball)) {
+      c->launches++;
+      return;
+    }
+  }
   dim3 grid((g.p1 - g.p0 + PB - 1) / PB, nfields);
   const size_t sm = smem_fft(2 * (g.nyp - 1), PB, sizeof(typename C2<T>::type));
-  // transform lengths 2(ny-1) of the production and test grids take the
+  // FP32: transform lengths 2(ny-1) of the production and test grids take the
   // compile-time plan
-  switch (2 * (g.nyp - 1)) {
-#define SB_CHEB_CASE(L)                                                                                      \
-  case L: {                                                                                                  \
-    constexpr int NT = fixed_threads(L, PB);                                                                 \
-    cudaFuncSetAttribute(k_cheb<T, PB, SI, SO, L, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm); \
-    k_cheb<T, PB, SI, SO, L, NT><<<grid, NT, sm, c->stream>>>(in, in_fs, out, out_fs, g, inverse, scale,      \
-                                                              c->twy.plan, tw, skip_oddball);               \
-    break;                                                                                                   \
-  }
+  switch (sizeof(T) == 8 ? 0 : 2 * (g.nyp - 1)) {
+#define SB_CHEB_CASE(L)                                                                                        \
+  case L:                                                                                                      \
+    if constexpr (sizeof(T) == 4) {                                                                            \
+      constexpr int NT = fixed_threads(L, PB);                                                                 \
+      cudaFuncSetAttribute(k_cheb<T, PB, SI, SO, L, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm); \
+      k_cheb<T, PB, SI, SO, L, NT><<<grid, NT, sm, c->stream>>>(in, in_fs, out, out_fs, g, inverse, scale,      \
+                                                                c->twy.plan, tw, skip_oddball);               \
+    }                                                                                                          \
+    break;
     SB_CHEB_CASE(128) SB_CHEB_CASE(192) SB_CHEB_CASE(256) SB_CHEB_CASE(384)
 #undef SB_CHEB_CASE
     default:
@@ -955,6 +963,37 @@ static void enqueue_sgs(sgpu_ctx* c) {
   launch_cheb_t<double, sgpu_ctx::pb, double, double>(c, czf(c, 6), fld, c->les_gu, fld, 3, 1, 1.0, 0, c->twy.d);
 }
 
+// FP64 step-2 passes of this context: the two-pass kernels (step2_f64.cuh) where
+// the length has one, the Stockham kernels with the runtime plan elsewhere.
+// in32: FP32 state (the pressure of a mixed run).
+static void zinv64(sgpu_ctx* c, const Dims& g, bool in32) {
+  if (f2_zinv(c->stream, c->st, in32 ? c->stf : nullptr, c->zb, g, c->twz.d, c->alfa, c->beta)) return;
+  const dim3 gz((g.nx2 + c->kb - 1) / c->kb, g.y1 - g.y0);
+  const size_t sm = smem_fft(g.nzp, c->kb, sizeof(double2));
+  if (in32)
+    launch_zinv<double, sgpu_ctx::kb, float>(gz, sm, c->stream, c->stf, c->zb, g, c->twz.plan, c->twz.d, c->alfa,
+                                             c->beta, 0);
+  else
+    launch_zinv<double, sgpu_ctx::kb, double>(gz, sm, c->stream, c->st, c->zb, g, c->twz.plan, c->twz.d, c->alfa,
+                                              c->beta, 0);
+}
+static void xpass64(sgpu_ctx* c, unsigned long long* cfl, Fringe fr) {
+  const Dims& g = c->g;
+  const sgpu_params& P = c->prm;
+  const double dxi = (double)(g.nx - 2) / P.xl, dzi = (double)(g.nz - 2) / P.zl;
+  if (f2_xpass(c->stream, c->zb, c->xb, g, c->twx.d, c->dyi, dxi, dzi, P.rot, cfl, fr)) return;
+  launch_xpass<double, sgpu_ctx::rb, sgpu_ctx::xpass64_threads>(
+      dim3((g.nzp + c->rb - 1) / c->rb, g.y1 - g.y0), smem_fft(g.nxp, 3 * c->rb, sizeof(double2)), c->stream, c->zb,
+      c->xb, g, c->twx.plan, c->twx.d, c->dyi, dxi, dzi, P.rot, cfl, nullptr, fr);
+}
+static void zfwd64(sgpu_ctx* c, const double2* in, double2* out) {
+  const Dims& g = c->g;
+  if (f2_zfwd(c->stream, in, out, g, c->twz.d)) return;
+  launch_zfwd<double, sgpu_ctx::kb, double>(dim3((g.nx2 + c->kb - 1) / c->kb, g.y1 - g.y0),
+                                            smem_fft(g.nzp, c->kb, sizeof(double2)), c->stream, in, out, g,
+                                            c->twz.plan, c->twz.d, nullptr, 0.0);
+}
+
 static int enqueue_nonlin(sgpu_ctx* c) {
   c->press_valid = false;
   NvtxRange nv("step 2 (nonlinbl)");
@@ -971,11 +1010,8 @@ static int enqueue_nonlin(sgpu_ctx* c) {
     c->launches++;
   }
   const int nyl = g.y1 - g.y0;  // this context's xz-planes
-  dim3 gz((g.nx2 + c->kb - 1) / c->kb, nyl);
-  const size_t s_z = smem_fft(g.nzp, c->kb, sizeof(double2));
   const double dxi = (double)(g.nx - 2) / P.xl;
   const double dzi = (double)(g.nz - 2) / P.zl;
-  const size_t s_x = smem_fft(g.nxp, 3 * c->rb, sizeof(double2));
   const size_t s_zf = smem_fft(g.nzp, sgpu_ctx::kbf, sizeof(float2));
   const size_t s_xf = smem_fft(g.nxp, 3 * sgpu_ctx::rbf, sizeof(float2));
   unsigned long long* cflp = do_cfl ? c->cfl_bits : nullptr;
@@ -998,16 +1034,11 @@ static int enqueue_nonlin(sgpu_ctx* c) {
     c->launches++;
   } else {
     prof_mark(c, K_ZINV);
-    launch_zinv<double, sgpu_ctx::kb, double>(gz, s_z, c->stream, c->st, c->zb, g, c->twz.plan, c->twz.d, c->alfa,
-                                              c->beta, 0);
-    dim3 gx((g.nzp + c->rb - 1) / c->rb, nyl);
+    zinv64(c, g, false);
     prof_mark(c, K_XPASS);
-    launch_xpass<double, sgpu_ctx::rb, sgpu_ctx::xpass64_threads>(gx, s_x, c->stream, c->zb, c->xb, g, c->twx.plan,
-                                                                  c->twx.d, c->dyi, dxi, dzi, P.rot, cflp, nullptr,
-                                                                  ctx_fringe(c));
+    xpass64(c, cflp, ctx_fringe(c));
     prof_mark(c, K_ZFWD);
-    launch_zfwd<double, sgpu_ctx::kb, double>(gz, s_z, c->stream, c->xb, c->st, g, c->twz.plan, c->twz.d, nullptr,
-                                              0.0);
+    zfwd64(c, c->xb, c->st);
   }
   c->launches += 3;
   if (c->iles >= 1) {
@@ -1219,14 +1250,8 @@ extern "C" int sgpu_cfl_rate(sgpu_ctx* c, double* rate) {
     mixed_xpass(c->stream, gxf, smem_fft(g.nxp, 3 * sgpu_ctx::rbf, sizeof(float2)), zbf, xbf, g, c->twx.plan,
                 c->twx.f, c->dyi, dxi, dzi, P.rot, c->cfl_bits, c->meanp, Fringe{nullptr, nullptr});
   } else {
-    dim3 gz((g.nx2 + c->kb - 1) / c->kb, nyl);
-    dim3 gx((g.nzp + c->rb - 1) / c->rb, nyl);
-    launch_zinv<double, sgpu_ctx::kb, double>(gz, smem_fft(g.nzp, c->kb, sizeof(double2)), c->stream, c->st, c->zb,
-                                              g, c->twz.plan, c->twz.d, c->alfa, c->beta, 0);
-    launch_xpass<double, sgpu_ctx::rb, sgpu_ctx::xpass64_threads>(gx, smem_fft(g.nxp, 3 * c->rb, sizeof(double2)),
-                                                                  c->stream, c->zb, c->xb, g, c->twx.plan, c->twx.d,
-                                                                  c->dyi, dxi, dzi, P.rot, c->cfl_bits, nullptr,
-                                                                  Fringe{nullptr, nullptr});
+    zinv64(c, g, false);
+    xpass64(c, c->cfl_bits, Fringe{nullptr, nullptr});
   }
   c->launches += c->mixed ? 4 : 3;
   CK(cudaGetLastError());
@@ -1798,22 +1823,15 @@ extern "C" int sgpu_pressure(sgpu_ctx* c, double* pr, double* pi) {
   }
   const sgpu_params& P = c->prm;
   // step-2 transforms of u, omega and the products H, 2E (nonlinp.f)
-  dim3 gz((g.nx2 + c->kb - 1) / c->kb, n);
-  const size_t s_z = smem_fft(g.nzp, c->kb, sizeof(double2));
-  if (c->mixed)
-    launch_zinv<double, sgpu_ctx::kb, float>(gz, s_z, c->stream, c->stf, c->zb, g, c->twz.plan, c->twz.d, c->alfa,
-                                             c->beta, 0);
-  else
-    launch_zinv<double, sgpu_ctx::kb, double>(gz, s_z, c->stream, c->st, c->zb, g, c->twz.plan, c->twz.d,
-                                              c->alfa, c->beta, 0);
-  const size_t s_xp = 2 * (size_t)g.nxp * 3 * sizeof(double2);
-  cudaFuncSetAttribute(k_xpass_p, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s_xp);
-  k_xpass_p<<<dim3(g.nzp, n), 256, s_xp, c->stream>>>(c->zb, g, c->twx.plan, c->twx.d, P.rot, ctx_fringe(c));
+  zinv64(c, g, c->mixed);
+  if (!f2_xpass_p(c->stream, c->zb, g, c->twx.d, P.rot, ctx_fringe(c))) {
+    const size_t s_xp = 2 * (size_t)g.nxp * 3 * sizeof(double2);
+    cudaFuncSetAttribute(k_xpass_p, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s_xp);
+    k_xpass_p<<<dim3(g.nzp, n), 256, s_xp, c->stream>>>(c->zb, g, c->twx.plan, c->twx.d, P.rot, ctx_fringe(c));
+  }
   const size_t fz = (size_t)n * g.nzp * g.nx2;  // one field of zb
-  launch_zfwd<double, sgpu_ctx::kb, double>(gz, s_z, c->stream, c->zb, czf(c, 0), g, c->twz.plan, c->twz.d,
-                                            nullptr, 0.0);  // H1, H2, H3
-  launch_zfwd<double, sgpu_ctx::kb, double>(gz, s_z, c->stream, c->zb + 3 * fz, czf(c, 3), g, c->twz.plan,
-                                            c->twz.d, nullptr, 0.0);  // 2E (fields 4, 5 overwritten below)
+  zfwd64(c, c->zb, czf(c, 0));           // H1, H2, H3
+  zfwd64(c, c->zb + 3 * fz, czf(c, 3));  // 2E (fields 4, 5 overwritten below)
   k_press_div<<<(unsigned)((fld + 255) / 256), 256, 0, c->stream>>>(czf(c, 0), g, c->alfa, c->beta);
   // Chebyshev coefficients (linearp.f:89-114)
   const double cn = 1.0 / ((double)g.nxp * (double)g.nzp);

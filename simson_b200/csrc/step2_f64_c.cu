@@ -1,0 +1,4 @@
+// Two-pass FP64 kernels of step 2, lengths SB_F2_LENGTHS_C (fft2.cuh).
+#define SB_F2_UNIT c
+#define SB_F2_UNIT_LENGTHS SB_F2_LENGTHS_C
+#include "step2_f64_unit.cuh"

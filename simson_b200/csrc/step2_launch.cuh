@@ -14,9 +14,10 @@ namespace sb {
 // threads per CTA of the runtime-plan FFT kernels
 constexpr int SB_FFT_THREADS = 256;
 
-// Transform lengths with compile-time FFT plans (fft.cuh cfft): the
+// FP32 transform lengths with compile-time FFT plans (fft.cuh cfft): the
 // production grid's 576 (3/2 x 384) and the test, LES and channel grids' 3/2
-// lengths; any other length takes the runtime plan.
+// lengths; any other length takes the runtime plan, and so do all FP64 ones
+// (those of step2_f64.cuh never come here).
 #define SB_FIXED_LENGTHS(X) X(72) X(96) X(240) X(288) X(576)
 
 // threads per CTA for B columns of an N-point compile-time transform: one
@@ -39,10 +40,11 @@ template <class T, int KB, class S>
 inline void launch_zinv(dim3 grid, size_t smem, cudaStream_t st, const typename C2<S>::type* in,
                         typename C2<T>::type* zb, const Dims& g, const FFTPlan& plan,
                         const typename C2<T>::type* tw, const double* alfa, const double* beta, int drop) {
-  switch (g.nzp) {
-#define SB_CASE(n)                                                                                 \
-  case n:                                                                                          \
-    zinv_n<T, KB, S, n, fixed_threads(n, KB)>(grid, smem, st, in, zb, g, plan, tw, alfa, beta, drop); \
+  switch (sizeof(T) == 8 ? 0 : g.nzp) {
+#define SB_CASE(n)                                                                                       \
+  case n:                                                                                                \
+    if constexpr (sizeof(T) == 4)                                                                        \
+      zinv_n<T, KB, S, n, fixed_threads(n, KB)>(grid, smem, st, in, zb, g, plan, tw, alfa, beta, drop);  \
     return;
     SB_FIXED_LENGTHS(SB_CASE)
 #undef SB_CASE
@@ -62,10 +64,11 @@ template <class T, int KB, class S>
 inline void launch_zfwd(dim3 grid, size_t smem, cudaStream_t st, const typename C2<T>::type* xb,
                         typename C2<S>::type* out, const Dims& g, const FFTPlan& plan,
                         const typename C2<T>::type* tw, const double* mean, double rot) {
-  switch (g.nzp) {
-#define SB_CASE(n)                                                                          \
-  case n:                                                                                   \
-    zfwd_n<T, KB, S, n, fixed_threads(n, KB)>(grid, smem, st, xb, out, g, plan, tw, mean, rot); \
+  switch (sizeof(T) == 8 ? 0 : g.nzp) {
+#define SB_CASE(n)                                                                                \
+  case n:                                                                                         \
+    if constexpr (sizeof(T) == 4)                                                                 \
+      zfwd_n<T, KB, S, n, fixed_threads(n, KB)>(grid, smem, st, xb, out, g, plan, tw, mean, rot); \
     return;
     SB_FIXED_LENGTHS(SB_CASE)
 #undef SB_CASE
@@ -90,11 +93,12 @@ inline void launch_xpass(dim3 grid, size_t smem, cudaStream_t st, const typename
                          typename C2<T>::type* xb, const Dims& g, const FFTPlan& plan,
                          const typename C2<T>::type* tw, const double* dyi, double dxi, double dzi, double rot,
                          unsigned long long* cfl, const double* mean, Fringe fr) {
-  switch (g.nxp) {
-#define SB_CASE(n)                                                                                        \
-  case n:                                                                                                 \
-    xpass_n<T, RB, n, fixed_threads(n, 3 * RB)>(grid, smem, st, zb, xb, g, plan, tw, dyi, dxi, dzi, rot, cfl, \
-                                                mean, fr);                                                \
+  switch (sizeof(T) == 8 ? 0 : g.nxp) {
+#define SB_CASE(n)                                                                                                \
+  case n:                                                                                                         \
+    if constexpr (sizeof(T) == 4)                                                                                 \
+      xpass_n<T, RB, n, fixed_threads(n, 3 * RB)>(grid, smem, st, zb, xb, g, plan, tw, dyi, dxi, dzi, rot, cfl,    \
+                                                  mean, fr);                                                      \
     return;
     SB_FIXED_LENGTHS(SB_CASE)
 #undef SB_CASE
