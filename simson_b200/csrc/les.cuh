@@ -3,18 +3,32 @@
 // bla/prhs.f:95-193) and the relaxation term -chi gu added to H in step 2
 // (bla/nonlinbl.f:920-965).  Filter tables: les_filter.h.
 //
-// One thread per (kx, kz) pencil and velocity component; the wall-normal
-// filter is a five-point right-hand side and a pentadiagonal LU solve along the
+// The tensorial filter (ihighorder = 2, the reference's default) applies the
+// wall-normal high pass N + 1 times to every column: a fixed ny x ny matrix
+// H_y^(N+1), built once, times all columns (k_les_hpf2).  The other modes: one
+// thread per (kx, kz) pencil and velocity component; the wall-normal filter is
+// a five-point right-hand side and a pentadiagonal LU solve along the
 // pencil, as the reference's hpf_y / lpf_y / pntdiag (bla/hpf_y.f,
 // bla/lpf_y.f, bla/bandsolver.f): a forward sweep (right-hand side from a
 // five-value register window, elimination) into a scratch column and a
 // backward substitution out of it.  Pencils are columns of stride NP, so a
 // warp reads 32 neighbouring complex values per row.
 #pragma once
+#include <vector>
+
 #include "fft.cuh"
 #include "layout.cuh"
 
 namespace sb {
+
+// Tile of k_les_hpf2: 16 pencils (32 real columns) by every row, eight rows
+// and two pencils per thread; the matrix in chunks of 16 columns
+constexpr int LES_TP = 16, LES_KC = 16;
+SB_HD __forceinline__ int les_hpf_ld(int n) { return (n + 7) / 8 * 8; }  // row length of the matrix, k-major
+inline int les_hpf_threads(int n) { return ((n + 7) / 8 * (LES_TP / 2) + 31) / 32 * 32; }
+inline int les_hpf_smem(int n) { return n * LES_TP * 16 + 2 * LES_KC * les_hpf_ld(n) * 8; }
+// whether the tile fits (ny up to about 800; the serial kernel serves the rest)
+inline bool les_hpf_fits(int n) { return les_hpf_smem(n) <= 227 * 1024 && les_hpf_threads(n) <= 1024; }
 
 // Per-row coefficients, LES_ROW doubles per row:
 //   [0..4]  right-hand-side stencil of the high pass (g2 - g1)
@@ -177,6 +191,23 @@ SB_HD __forceinline__ void les_hpf_column(const YFilter& F, int mode, int iord, 
   }
 }
 
+// H_y^(N+1) as k_les_hpf2 reads it: two unit vectors at a time through the
+// column filter.
+inline void les_hpf_matrix(const YFilter& F, int iord, std::vector<double>& M) {
+  const int n = F.n, ld = les_hpf_ld(n);
+  M.assign((size_t)n * ld, 0.0);
+  std::vector<double2> u(n), z(n);
+  for (int k = 0; k < n; k += 2) {
+    for (int j = 0; j < n; ++j) u[j] = double2{j == k ? 1.0 : 0.0, j == k + 1 ? 1.0 : 0.0};
+    for (int it = 0; it <= iord; ++it)
+      yfilter_column(F, true, [&](int j) { return u[j]; }, z.data(), 1, [&](int j, double2 x) { u[j] = x; });
+    for (int j = 0; j < n; ++j) {
+      M[(size_t)k * ld + j] = u[j].x;
+      if (k + 1 < n) M[(size_t)(k + 1) * ld + j] = u[j].y;
+    }
+  }
+}
+
 #ifdef __CUDACC__
 // gu[ll] for ll = blockIdx.y (0..2) from the velocity slots of st (FP64 or
 // FP32 storage); one thread per pencil.  skip_oddball leaves the kz = -nz/2
@@ -192,6 +223,92 @@ __global__ void __launch_bounds__(128) k_les_hpf(const V* __restrict__ st, doubl
   const int ll = blockIdx.y;
   les_hpf_column(F, mode, iord, lpf[p], filt[p], st + ll * fld + p, gu + ll * fld + p, Z + ll * fld + p,
                  (size_t)g.NP);
+}
+
+// gu = u - L_xz (u - H u), H = H_y^(N+1) as the matrix M[k][j] (row k holds
+// column k of H, les_hpf_ld(n) long), for fields blockIdx.y.  A product of
+// n x n by all 2 NP columns: each thread keeps eight rows of two pencils (32
+// accumulators), the tile's u in shared memory, M through two chunk buffers
+// filled asynchronously (read row by row from L2 instead, each row waited a
+// round trip: 57 us at 64x97x64).  FP64-bound: 2 n^2 flops per column; the
+// serial column solves (six forward and backward sweeps of one thread per
+// pencil, 48 CTAs) took 284 us there.
+template <class V>
+__global__ void k_les_hpf2(const V* __restrict__ st, double2* __restrict__ gu, const double* __restrict__ M,
+                           const double* __restrict__ lpf, Dims g, int skip_oddball) {
+  extern __shared__ __align__(16) unsigned char les_smem[];
+  double2* U = reinterpret_cast<double2*>(les_smem);  // [n][LES_TP]
+  const int n = g.nyp, ld = les_hpf_ld(n);
+  const size_t fld = (size_t)n * g.NP;
+  const int p0 = blockIdx.x * LES_TP;
+  const V* __restrict__ src = st + blockIdx.y * fld;
+  double2* __restrict__ dst = gu + blockIdx.y * fld;
+  for (int i = threadIdx.x; i < n * LES_TP; i += blockDim.x) {
+    const int p = p0 + i % LES_TP;
+    U[i] = p < g.NP ? to_d2(src[(size_t)(i / LES_TP) * g.NP + p]) : double2{0.0, 0.0};
+  }
+  __syncthreads();
+  double2* const buf = U + n * LES_TP;  // [2][LES_KC][ld / 2]
+  const int ld2 = ld / 2;
+  const double2* __restrict__ m = reinterpret_cast<const double2*>(M);
+  auto fetch = [&](int k0, int b) {
+    const int cnt = min(LES_KC, n - k0) * ld2;
+    for (int i = threadIdx.x; i < cnt; i += blockDim.x) {
+      const unsigned d = (unsigned)__cvta_generic_to_shared(&buf[b * LES_KC * ld2 + i]);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(m + (size_t)k0 * ld2 + i) : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  fetch(0, 0);
+  const int q = (threadIdx.x % (LES_TP / 2)) * 2, j0 = threadIdx.x / (LES_TP / 2) * 8;
+  const bool work = j0 < n;
+  double2 a[8][2];
+#pragma unroll
+  for (int r = 0; r < 8; ++r) a[r][0] = a[r][1] = double2{0.0, 0.0};
+  for (int k0 = 0, b = 0; k0 < n; k0 += LES_KC, b ^= 1) {
+    if (k0 + LES_KC < n) {
+      fetch(k0 + LES_KC, b ^ 1);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+    }
+    __syncthreads();
+    if (work) {
+      const double2* hb = buf + b * LES_KC * ld2 + j0 / 2;
+      const int kn = min(LES_KC, n - k0);
+#pragma unroll 4
+      for (int k = 0; k < kn; ++k) {
+        const double2 u0 = U[(k0 + k) * LES_TP + q], u1 = U[(k0 + k) * LES_TP + q + 1];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          const double2 h = hb[k * ld2 + r];
+          a[2 * r][0].x = fma_(h.x, u0.x, a[2 * r][0].x);
+          a[2 * r][0].y = fma_(h.x, u0.y, a[2 * r][0].y);
+          a[2 * r][1].x = fma_(h.x, u1.x, a[2 * r][1].x);
+          a[2 * r][1].y = fma_(h.x, u1.y, a[2 * r][1].y);
+          a[2 * r + 1][0].x = fma_(h.y, u0.x, a[2 * r + 1][0].x);
+          a[2 * r + 1][0].y = fma_(h.y, u0.y, a[2 * r + 1][0].y);
+          a[2 * r + 1][1].x = fma_(h.y, u1.x, a[2 * r + 1][1].x);
+          a[2 * r + 1][1].y = fma_(h.y, u1.y, a[2 * r + 1][1].y);
+        }
+      }
+    }
+    __syncthreads();  // before the next fetch overwrites this buffer
+  }
+  if (!work) return;
+#pragma unroll
+  for (int s = 0; s < 2; ++s) {
+    const int p = p0 + q + s;
+    if (p >= g.NP || (skip_oddball && p / g.nx2 == g.zodd)) continue;
+    const double l = lpf[p];
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      if (j0 + r >= n) break;
+      const double2 u = U[(j0 + r) * LES_TP + q + s];
+      dst[(size_t)(j0 + r) * g.NP + p] =
+          double2{u.x - l * (u.x - a[r][s].x), u.y - l * (u.y - a[r][s].y)};
+    }
+  }
 }
 
 // H_ll -= chi gu_ll nxp nzp on the stored modes, the oddball plane excepted

@@ -120,6 +120,7 @@ struct sgpu_ctx {
   double* les_coef = nullptr;  // [nyp][LES_ROW]
   double* les_lpf = nullptr;   // [NP] L_xz
   double* les_filt = nullptr;  // [NP] F_xz
+  double* les_hmat = nullptr;  // H_y^(N+1) (k_les_hpf2), mode 2
   double les_fact2 = 0.0, les_factm2 = 0.0;
   // eddy-viscosity LES (iles = 2): buffers on the unpadded nx x nz grid
   SgsBufs sgs{};
@@ -531,7 +532,7 @@ extern "C" int sgpu_finalize(sgpu_ctx* c) {
   if (!c) return SGPU_OK;
   if (c->stream) cudaStreamSynchronize(c->stream);
   if (c->step_exec) cudaGraphExecDestroy(c->step_exec);
-  void* ptrs[] = {c->st, c->stf, c->meanp, c->ampd, c->les_gu, c->les_coef, c->les_lpf, c->les_filt,
+  void* ptrs[] = {c->st, c->stf, c->meanp, c->ampd, c->les_gu, c->les_coef, c->les_lpf, c->les_filt, c->les_hmat,
                   c->sgs.spec9, c->sgs.phys10, c->sgs.filt21, c->sgs.numden, c->sgs.cxy, c->sgs.tauz6, c->sgs.tau,
                   c->sgs_delta2, c->sgs_twz.d, c->sgs_twz.f, c->sgs_twx.d, c->sgs_twx.f, c->xys, c->xys_spec,
                   c->xys_part, c->xys_u, c->box_out, c->press, c->press_wd, c->xys_twz.d, c->xys_twz.f, c->xys_twx.d, c->xys_twx.f, c->mlp_image, c->mlp_tau,
@@ -830,26 +831,31 @@ extern "C" int sgpu_prhs(sgpu_ctx* c) {
 static void les_filter_velocity(sgpu_ctx* c, int skip_oddball) {
   const Dims& g = c->g;
   YFilter F{c->les_coef, c->les_fact2, c->les_factm2, g.nyp};
-  dim3 grid((g.NP + 127) / 128, c->iles == 3 ? 5 : 3);
+  const int nf = c->iles == 3 ? 5 : 3;
   prof_mark(c, K_OTHER);
-  if (c->mixed)
-    k_les_hpf<float2><<<grid, 128, 0, c->stream>>>(c->stf, c->les_gu, czf(c, 0), F, c->les_lpf, c->les_filt, g,
-                                                   c->les_mode, c->les_iord, skip_oddball);
-  else
-    k_les_hpf<double2><<<grid, 128, 0, c->stream>>>(c->st, c->les_gu, czf(c, 0), F, c->les_lpf, c->les_filt, g,
-                                                    c->les_mode, c->les_iord, skip_oddball);
-  c->launches++;
-  if (c->iles == 3 && c->hpf_dyn) {
-    // the secondary filter (bla/linearbl.f:2067-2250, the same wall-normal
-    // filter, the x/z tables of the quarter cut-off) for the dynamic procedure
-    if (c->mixed)
-      k_les_hpf<float2><<<grid, 128, 0, c->stream>>>(c->stf, c->les_gu2, czf(c, 0), F, c->les_lpf2, c->les_filt2, g,
-                                                     c->les_mode, c->les_iord, skip_oddball);
-    else
-      k_les_hpf<double2><<<grid, 128, 0, c->stream>>>(c->st, c->les_gu2, czf(c, 0), F, c->les_lpf2, c->les_filt2,
-                                                      g, c->les_mode, c->les_iord, skip_oddball);
+  auto filter = [&](double2* gu, const double* lpf, const double* filt) {
+    if (c->les_mode == 2 && les_hpf_fits(g.nyp)) {
+      const dim3 grid((g.NP + LES_TP - 1) / LES_TP, nf);
+      const int nt = les_hpf_threads(g.nyp), sm = les_hpf_smem(g.nyp);
+      if (c->mixed)
+        k_les_hpf2<float2><<<grid, nt, sm, c->stream>>>(c->stf, gu, c->les_hmat, lpf, g, skip_oddball);
+      else
+        k_les_hpf2<double2><<<grid, nt, sm, c->stream>>>(c->st, gu, c->les_hmat, lpf, g, skip_oddball);
+    } else {
+      const dim3 grid((g.NP + 127) / 128, nf);
+      if (c->mixed)
+        k_les_hpf<float2><<<grid, 128, 0, c->stream>>>(c->stf, gu, czf(c, 0), F, lpf, filt, g, c->les_mode,
+                                                       c->les_iord, skip_oddball);
+      else
+        k_les_hpf<double2><<<grid, 128, 0, c->stream>>>(c->st, gu, czf(c, 0), F, lpf, filt, g, c->les_mode,
+                                                        c->les_iord, skip_oddball);
+    }
     c->launches++;
-  }
+  };
+  filter(c->les_gu, c->les_lpf, c->les_filt);
+  // the secondary filter (bla/linearbl.f:2067-2250, the same wall-normal
+  // filter, the x/z tables of the quarter cut-off) for the dynamic procedure
+  if (c->iles == 3 && c->hpf_dyn) filter(c->les_gu2, c->les_lpf2, c->les_filt2);
 }
 
 static SgsGrid sgs_grid(const sgpu_ctx* c) {
@@ -2248,6 +2254,21 @@ extern "C" int sgpu_set_les(sgpu_ctx* c, const sgpu_les_params* p) {
   CK(cudaMemcpyAsync(c->les_filt, F.filtxz.data(), (size_t)g.NP * sizeof(double), cudaMemcpyHostToDevice,
                      c->stream));
   CK(cudaStreamSynchronize(c->stream));
+  if (p->ihighorder == 2 && les_hpf_fits(g.nyp)) {
+    // the wall-normal matrix of the tensorial filter
+    YFilter Y{rows.data(), F.fact2, F.factm2, g.nyp};
+    std::vector<double> M;
+    les_hpf_matrix(Y, p->iord, M);
+    if (!c->les_hmat && cudaMalloc(&c->les_hmat, M.size() * sizeof(double)) != cudaSuccess) {
+      c->les_hmat = nullptr;  // (the matrix's size depends on ny only)
+      return SGPU_E_CUDA;
+    }
+    CK(cudaMemcpyAsync(c->les_hmat, M.data(), M.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
+    const int sm = les_hpf_smem(g.nyp);
+    cudaFuncSetAttribute(k_les_hpf2<float2>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+    cudaFuncSetAttribute(k_les_hpf2<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+  }
   c->les_fact2 = F.fact2;
   c->les_factm2 = F.factm2;
   c->les_mode = p->ihighorder;
