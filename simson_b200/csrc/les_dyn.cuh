@@ -183,7 +183,7 @@ __device__ __forceinline__ double sgs_sabs(const double* s) {
 // s2 != nullptr: the test filter's B_ij parts are these six physical fields
 // (the dynamic HPF model: the strain of the secondary high-pass filtered
 // field, bla/les.f:1031-1250) instead of S_ij.
-__global__ void k_sgs_xpass1(SgsBufs B, SgsGrid G, FFTPlan plan, const double2* __restrict__ tw,
+static __global__ void k_sgs_xpass1(SgsBufs B, SgsGrid G, FFTPlan plan, const double2* __restrict__ tw,
                              const double* __restrict__ delta2, const double* __restrict__ s2) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int NC = 11;
@@ -255,7 +255,7 @@ __global__ void k_sgs_xpass1(SgsBufs B, SgsGrid G, FFTPlan plan, const double2* 
 // The nine spec9 rows of one z row back to physical x: fields f0..8 into
 // out[f - f0] (the learned model's gradients: out = phys10, f0 = 0; the
 // dynamic HPF model's secondary strain: f0 = 3).
-__global__ void k_sgs_xinv9(SgsBufs B, SgsGrid G, FFTPlan plan, const double2* __restrict__ tw,
+static __global__ void k_sgs_xinv9(SgsBufs B, SgsGrid G, FFTPlan plan, const double2* __restrict__ tw,
                             double* __restrict__ out, int f0) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double2* bA = reinterpret_cast<double2*>(smem_raw);
@@ -319,9 +319,29 @@ __global__ void k_sgs_zfilt(SgsBufs B, SgsGrid G, FFTPlan plan, const double2* _
   }
 }
 
+// Per-point contractions M:L and M:M (les.f:783-881) of the 21 test-filtered
+// values r: M parts, -u_i u_j, S_ij, u_i; gd2 = 4^(2/3) Delta^2.
+__device__ __forceinline__ void sgs_germano(const double* r, double gd2, double& num, double& den) {
+  const double* mt = r;       // filtered M parts
+  const double* lt = r + 6;   // filtered -u_i u_j
+  const double* bt = r + 12;  // filtered S
+  const double u = r[18], v = r[19], w = r[20];
+  double L[6], M[6];
+  L[0] = lt[0] + u * u;
+  L[1] = lt[1] + v * u;
+  L[2] = lt[2] + w * u;
+  L[3] = lt[3] + v * v;
+  L[4] = lt[4] + w * v;
+  L[5] = lt[5] + w * w;
+  const double dr = gd2 * sgs_sabs(bt);
+  for (int l = 0; l < 6; ++l) M[l] = mt[l] + bt[l] * dr;
+  num = M[0] * L[0] + M[3] * L[3] + M[5] * L[5] + 2. * (M[1] * L[1] + M[2] * L[2] + M[4] * L[4]);
+  den = M[0] * M[0] + M[3] * M[3] + M[5] * M[5] + 2. * (M[1] * M[1] + M[2] * M[2] + M[4] * M[4]);
+}
+
 // Inverse x FFT of the 21 test-filtered fields (divided by nx nz as
 // filter_cutoff.f does), then L_ij, M_ij and the per-point contractions.
-__global__ void k_sgs_xpass2(SgsBufs B, SgsGrid G, FFTPlan plan, const double2* __restrict__ tw,
+static __global__ void k_sgs_xpass2(SgsBufs B, SgsGrid G, FFTPlan plan, const double2* __restrict__ tw,
                              const double* __restrict__ delta2) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int NC = 11;
@@ -352,21 +372,8 @@ __global__ void k_sgs_xpass2(SgsBufs B, SgsGrid G, FFTPlan plan, const double2* 
       r[2 * c] = z.x * inv;
       r[2 * c + 1] = z.y * inv;
     }
-    const double* mt = r;       // filtered M parts
-    const double* lt = r + 6;   // filtered -u_i u_j
-    const double* bt = r + 12;  // filtered S
-    const double u = r[18], v = r[19], w = r[20];
-    double L[6], M[6];
-    L[0] = lt[0] + u * u;
-    L[1] = lt[1] + v * u;
-    L[2] = lt[2] + w * u;
-    L[3] = lt[3] + v * v;
-    L[4] = lt[4] + w * v;
-    L[5] = lt[5] + w * w;
-    const double dr = gd2 * sgs_sabs(bt);
-    for (int l = 0; l < 6; ++l) M[l] = mt[l] + bt[l] * dr;
-    const double num = M[0] * L[0] + M[3] * L[3] + M[5] * L[5] + 2. * (M[1] * L[1] + M[2] * L[2] + M[4] * L[4]);
-    const double den = M[0] * M[0] + M[3] * M[3] + M[5] * M[5] + 2. * (M[1] * M[1] + M[2] * M[2] + M[4] * M[4]);
+    double num, den;
+    sgs_germano(r, gd2, num, den);
     B.numden[prow + j] = num;
     B.numden[fs10 + prow + j] = den;
   }
@@ -375,20 +382,35 @@ __global__ void k_sgs_xpass2(SgsBufs B, SgsGrid G, FFTPlan plan, const double2* 
 // C(x, y) from the z averages (les.f:1385-1480).  cs > 0: fixed C = cs^2.
 // ineg: 0 no clipping, 1 C >= 0 and zero at the walls, 2 zero at the walls
 // (the nu_t + nu >= 0 clip follows in k_sgs_tau_x).
-__global__ void k_sgs_coef(SgsBufs B, SgsGrid G, double cs, int ineg) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
+// 32 x points per CTA, SGS_CZ z groups summed in shared memory: one thread per
+// x point walked nz strided loads alone (35 us at 64x97x64).
+constexpr int SGS_CZ = 8;
+static __global__ void __launch_bounds__(32 * SGS_CZ) k_sgs_coef(SgsBufs B, SgsGrid G, double cs, int ineg) {
+  __shared__ double sn[SGS_CZ][32], sd[SGS_CZ][32];
+  const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5;
+  const int x = blockIdx.x * 32 + lane;
   const int y = blockIdx.y;
-  if (x >= G.nx || sgs_plane_off(B, y)) return;
+  if (sgs_plane_off(B, y)) return;  // the whole CTA
+  double num = 0.0, den = 0.0;
+  if (cs == 0.0 && x < G.nx) {
+    const size_t plane = (size_t)G.nyp * G.nz * G.nx;
+    for (int m = grp; m < G.nz; m += SGS_CZ) {
+      const size_t o = ((size_t)y * G.nz + m) * G.nx + x;
+      num += B.numden[o];
+      den += B.numden[plane + o];
+    }
+  }
+  sn[grp][lane] = num;
+  sd[grp][lane] = den;
+  __syncthreads();
+  if (grp != 0 || x >= G.nx) return;
   double c;
   if (cs != 0.0) {
     c = cs * cs;
   } else {
-    const size_t plane = (size_t)G.nyp * G.nz * G.nx;
-    double num = 0.0, den = 0.0;
-    for (int m = 0; m < G.nz; ++m) {
-      const size_t o = ((size_t)y * G.nz + m) * G.nx + x;
-      num += B.numden[o];
-      den += B.numden[plane + o];
+    for (int i = 1; i < SGS_CZ; ++i) {
+      num += sn[i][lane];
+      den += sd[i][lane];
     }
     const bool wall = (y == 0 || y == G.nyp - 1);
     if (ineg == 1)
@@ -401,12 +423,30 @@ __global__ void k_sgs_coef(SgsBufs B, SgsGrid G, double cs, int ineg) {
   B.cxy[(size_t)y * G.nx + x] = c;
 }
 
+// tau_ij / (nx nz) at point j of a row: the given physical stress, or the
+// eddy-viscosity one (tau_phys == nullptr)
+__device__ __forceinline__ void sgs_tau_point(const SgsBufs& B, const SgsGrid& G, double d2, double re, int ineg,
+                                              const double* __restrict__ tau_phys, size_t fs10, size_t prow, int y,
+                                              int j, double (&t)[6]) {
+  const double gd2 = 1. / (double)(G.nx * G.nz);
+  if (tau_phys != nullptr) {
+#pragma unroll
+    for (int l = 0; l < 6; ++l) t[l] = tau_phys[(size_t)l * fs10 + prow + j] * gd2;
+    return;
+  }
+  double dr = B.cxy[(size_t)y * G.nx + j] * B.phys10[9 * fs10 + prow + j] * d2;
+  if (ineg == 2 && dr < -1. / re) dr = -1. / re;
+  const double d1 = -2. * dr * gd2;
+#pragma unroll
+  for (int l = 0; l < 6; ++l) t[l] = d1 * B.phys10[(size_t)(3 + l) * fs10 + prow + j];
+}
+
 // tau_ij / (nx nz) = -2 C Delta^2 |S| S_ij / (nx nz) in physical space, then
 // the forward x FFT (three complex FFTs for the six real rows).
 // tau_phys != nullptr: the stress is given in physical space ([6][nyp*nz*nx],
 // the learned model) instead of -2 C Delta^2 |S| S_ij, except on the planes
 // that B.plane_on switches to the eddy-viscosity model.
-__global__ void k_sgs_tau_x(SgsBufs B, SgsGrid G, FFTPlan plan, const double2* __restrict__ tw,
+static __global__ void k_sgs_tau_x(SgsBufs B, SgsGrid G, FFTPlan plan, const double2* __restrict__ tw,
                             const double* __restrict__ delta2, double re, int ineg,
                             const double* __restrict__ tau_phys) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -416,19 +456,11 @@ __global__ void k_sgs_tau_x(SgsBufs B, SgsGrid G, FFTPlan plan, const double2* _
   const int n = G.nx;
   const size_t fs10 = (size_t)G.nyp * G.nz * G.nx;
   const size_t prow = ((size_t)y * G.nz + m) * G.nx;
-  const double gd2 = 1. / (double)(G.nx * G.nz);
   const double d2 = delta2[y];
   const bool learned = tau_phys != nullptr && (B.plane_on == nullptr || B.plane_on[y] == 0);
   for (int j = threadIdx.x; j < n; j += blockDim.x) {
     double t[6];
-    if (learned) {
-      for (int l = 0; l < 6; ++l) t[l] = tau_phys[(size_t)l * fs10 + prow + j] * gd2;
-    } else {
-      double dr = B.cxy[(size_t)y * G.nx + j] * B.phys10[9 * fs10 + prow + j] * d2;
-      if (ineg == 2 && dr < -1. / re) dr = -1. / re;
-      const double d1 = -2. * dr * gd2;
-      for (int l = 0; l < 6; ++l) t[l] = d1 * B.phys10[(size_t)(3 + l) * fs10 + prow + j];
-    }
+    sgs_tau_point(B, G, d2, re, ineg, learned ? tau_phys : nullptr, fs10, prow, y, j, t);
     for (int c = 0; c < 3; ++c) bA[j * 3 + c] = double2{t[2 * c], t[2 * c + 1]};
   }
   __syncthreads();
@@ -453,7 +485,7 @@ __global__ void k_sgs_tau_x(SgsBufs B, SgsGrid G, FFTPlan plan, const double2* _
 // plane switches to the eddy-viscosity model when sum P > bound * sum |P|
 // (bound in [-1, 1]: 1 never, below -1 always).  sums[2 y], sums[2 y + 1]
 // keep the two sums for diagnostics.
-__global__ void __launch_bounds__(1024) k_sgs_backscatter(SgsBufs B, SgsGrid G, const double* __restrict__ tau,
+static __global__ void __launch_bounds__(1024) k_sgs_backscatter(SgsBufs B, SgsGrid G, const double* __restrict__ tau,
                                                          double bound, int* __restrict__ plane_on,
                                                          double* __restrict__ sums) {
   const int y = blockIdx.x;
@@ -534,7 +566,7 @@ __global__ void k_sgs_zfwd(SgsBufs B, SgsGrid G, FFTPlan plan, const double2* __
 // closed form of the bla/dcheb.f recurrence) -- as suffix sums: each lane
 // sums its block of rows by parity, the warp scans the block sums, and each
 // lane walks its rows down from its carry.
-__global__ void __launch_bounds__(128) k_sgs_sigma(const double2* __restrict__ tc, double2* __restrict__ sc,
+static __global__ void __launch_bounds__(128) k_sgs_sigma(const double2* __restrict__ tc, double2* __restrict__ sc,
                                                    SgsGrid G, const double* __restrict__ alfa,
                                                    const double* __restrict__ beta) {
   const int lane = threadIdx.x & 31;

@@ -29,6 +29,7 @@
 #include "mixed.h"
 #include "step2_launch.cuh"
 #include "step2_f64.h"
+#include "les_f64.h"
 #include "cheb_tc.cuh"
 #include "pencil_chunk.h"
 #include "pencil_warp.cuh"
@@ -871,44 +872,49 @@ static void enqueue_sgs(sgpu_ctx* c) {
   constexpr int KB = 4;
   const size_t sz = 2 * (size_t)g.nz * KB * sizeof(double2);
   const size_t sx11 = 2 * (size_t)g.nx * 11 * sizeof(double2);
+  const size_t sx5 = 2 * (size_t)g.nx * 5 * sizeof(double2);
   const size_t sx3 = 2 * (size_t)g.nx * 3 * sizeof(double2);
   prof_mark(c, K_OTHER);
-  dim3 gz((g.nx2 + KB - 1) / KB, g.nyp), gz4((G.nx4 + KB - 1) / KB, g.nyp), gx(g.nz, g.nyp);
-  const int set = (c->iles == 4) ? 1 : 0;
-  const double* s2 = nullptr;
-  if (c->iles == 3 && c->hpf_dyn) {
-    // dynamic HPF (bla/les.f:968-1383): first the strain of the secondary
-    // filtered field in physical space (test-filtered below in place of S),
-    // then u of the state with the strain of the primary filtered field
-    k_sgs_zinv<double2, KB><<<gz, 256, sz, c->stream>>>(c->les_gu2, c->sgs, G, c->sgs_twz.plan, c->sgs_twz.d,
-                                                        c->alfa, c->beta, 0, nullptr);
-    k_sgs_xinv9<<<gx, 128, 2 * (size_t)g.nx * 5 * sizeof(double2), c->stream>>>(c->sgs, G, c->sgs_twx.plan,
-                                                                                 c->sgs_twx.d, c->hpf_s2, 3);
-    s2 = c->hpf_s2;
-    c->launches += 2;
-    if (c->mixed)
-      k_sgs_zinv<float2, KB><<<gz, 256, sz, c->stream>>>(c->stf, c->sgs, G, c->sgs_twz.plan, c->sgs_twz.d, c->alfa,
-                                                         c->beta, 0, c->les_gu);
+  const dim3 gz((g.nx2 + KB - 1) / KB, g.nyp), gz4((G.nx4 + KB - 1) / KB, g.nyp), gx(g.nz, g.nyp);
+  const FFTPlan &pz = c->sgs_twz.plan, &px = c->sgs_twx.plan;
+  const double2 *tz = c->sgs_twz.d, *tx = c->sgs_twx.d;
+  cudaStream_t st = c->stream;
+  // each pass: the two-pass kernel of its length, or the one with the runtime plan
+  auto zinv = [&](const SgsBufs& B, const double2* src, const float2* srcf, int set, const double2* sf) {
+    c->launches++;
+    if (lf_zinv(st, src, srcf, B, G, tz, c->alfa, c->beta, set, sf)) return;
+    if (srcf)
+      k_sgs_zinv<float2, KB><<<gz, 256, sz, st>>>(srcf, B, G, pz, tz, c->alfa, c->beta, set, sf);
     else
-      k_sgs_zinv<double2, KB><<<gz, 256, sz, c->stream>>>(c->st, c->sgs, G, c->sgs_twz.plan, c->sgs_twz.d, c->alfa,
-                                                          c->beta, 0, c->les_gu);
-  } else if (c->iles == 3) {
-    // HPF model, fixed constant: the strain of the high-pass filtered fields
-    // (bla/les.f:404-450, 883-966)
-    k_sgs_zinv<double2, KB><<<gz, 256, sz, c->stream>>>(c->les_gu, c->sgs, G, c->sgs_twz.plan, c->sgs_twz.d,
-                                                        c->alfa, c->beta, 0, nullptr);
-  } else if (c->mixed) {
-    k_sgs_zinv<float2, KB><<<gz, 256, sz, c->stream>>>(c->stf, c->sgs, G, c->sgs_twz.plan, c->sgs_twz.d, c->alfa,
-                                                       c->beta, set, nullptr);
-  } else {
-    k_sgs_zinv<double2, KB><<<gz, 256, sz, c->stream>>>(c->st, c->sgs, G, c->sgs_twz.plan, c->sgs_twz.d, c->alfa,
-                                                        c->beta, set, nullptr);
-  }
+      k_sgs_zinv<double2, KB><<<gz, 256, sz, st>>>(src, B, G, pz, tz, c->alfa, c->beta, set, sf);
+  };
+  auto state_zinv = [&](const SgsBufs& B, int set, const double2* sf) {
+    zinv(B, c->st, c->mixed ? c->stf : nullptr, set, sf);
+  };
+  auto xinv9 = [&](double* out, int f0) {
+    c->launches++;
+    if (!lf_xinv9(st, c->sgs, G, tx, out, f0)) k_sgs_xinv9<<<gx, 128, sx5, st>>>(c->sgs, G, px, tx, out, f0);
+  };
+  // the dynamic coefficient from the transformed strain of B's spec9
+  auto coefficient = [&](const SgsBufs& B, const double* s2) {
+    if (!lf_xpass1(st, B, G, tx, c->sgs_delta2, s2))
+      k_sgs_xpass1<<<gx, 128, sx11, st>>>(B, G, px, tx, c->sgs_delta2, s2);
+    if (!lf_zfilt(st, B, G, tz)) k_sgs_zfilt<KB><<<gz4, 256, sz, st>>>(B, G, pz, tz);
+    if (!lf_xpass2(st, B, G, tx, c->sgs_delta2)) k_sgs_xpass2<<<gx, 128, sx11, st>>>(B, G, px, tx, c->sgs_delta2);
+    k_sgs_coef<<<dim3((g.nx + 31) / 32, g.nyp), 32 * SGS_CZ, 0, st>>>(B, G, c->les_cs, c->les_ineg);
+    c->launches += 4;
+  };
+  auto stress = [&](const SgsBufs& B, const double* tau_phys) {
+    if (!lf_tau_x(st, B, G, tx, c->sgs_delta2, c->prm.re, c->les_ineg, tau_phys))
+      k_sgs_tau_x<<<gx, 128, sx3, st>>>(B, G, px, tx, c->sgs_delta2, c->prm.re, c->les_ineg, tau_phys);
+    if (!lf_zfwd(st, c->sgs, G, tz)) k_sgs_zfwd<KB><<<gz, 256, sz, st>>>(c->sgs, G, pz, tz);
+    c->launches += 2;
+  };
   if (c->iles == 4) {
     // learned model: gradients to physical space, MLP on the tensor cores,
     // tau / (nx nz) back to Fourier space
-    k_sgs_xinv9<<<gx, 128, 2 * (size_t)g.nx * 5 * sizeof(double2), c->stream>>>(c->sgs, G, c->sgs_twx.plan,
-                                                                                 c->sgs_twx.d, c->sgs.phys10, 0);
+    state_zinv(c->sgs, 1, nullptr);
+    xinv9(c->sgs.phys10, 0);
     MlpArgs A{};
     A.image = c->mlp_image;
     A.mode = 1;
@@ -925,40 +931,38 @@ static void enqueue_sgs(sgpu_ctx* c) {
     A.test_timeout = c->test_timeout;
     const long long tiles = (A.n + MLP_ROWS - 1) / MLP_ROWS;
     const int blocks = (int)std::min<long long>(tiles, 148 * 4);
-    k_sgs_mlp<<<blocks, 128, MLP_SMEM_LAUNCH, c->stream>>>(A);
-    c->launches += 2;
+    k_sgs_mlp<<<blocks, 128, MLP_SMEM_LAUNCH, st>>>(A);
+    c->launches++;
     SgsBufs F = c->sgs;
     if (c->sgs_fb) {
       // per-plane fallback: planes whose predicted backscatter exceeds the
       // bound take the eddy-viscosity stress (its kernels skip the others)
-      k_sgs_backscatter<<<g.nyp, 1024, 0, c->stream>>>(c->sgs, G, c->mlp_tau, c->sgs_fb_bound, c->sgs_flags,
-                                                       c->sgs_bsums);
+      k_sgs_backscatter<<<g.nyp, 1024, 0, st>>>(c->sgs, G, c->mlp_tau, c->sgs_fb_bound, c->sgs_flags, c->sgs_bsums);
+      c->launches++;
       F.plane_on = c->sgs_flags;
-      if (c->mixed)
-        k_sgs_zinv<float2, KB><<<gz, 256, sz, c->stream>>>(c->stf, F, G, c->sgs_twz.plan, c->sgs_twz.d, c->alfa,
-                                                           c->beta, 0, nullptr);
-      else
-        k_sgs_zinv<double2, KB><<<gz, 256, sz, c->stream>>>(c->st, F, G, c->sgs_twz.plan, c->sgs_twz.d, c->alfa,
-                                                            c->beta, 0, nullptr);
-      k_sgs_xpass1<<<gx, 128, sx11, c->stream>>>(F, G, c->sgs_twx.plan, c->sgs_twx.d, c->sgs_delta2, nullptr);
-      k_sgs_zfilt<KB><<<gz4, 256, sz, c->stream>>>(F, G, c->sgs_twz.plan, c->sgs_twz.d);
-      k_sgs_xpass2<<<gx, 128, sx11, c->stream>>>(F, G, c->sgs_twx.plan, c->sgs_twx.d, c->sgs_delta2);
-      k_sgs_coef<<<dim3((g.nx + 127) / 128, g.nyp), 128, 0, c->stream>>>(F, G, c->les_cs, c->les_ineg);
-      c->launches += 6;
+      state_zinv(F, 0, nullptr);
+      coefficient(F, nullptr);
     }
-    k_sgs_tau_x<<<gx, 128, sx3, c->stream>>>(F, G, c->sgs_twx.plan, c->sgs_twx.d, c->sgs_delta2, c->prm.re,
-                                             c->les_ineg, c->mlp_tau);
-    k_sgs_zfwd<KB><<<gz, 256, sz, c->stream>>>(c->sgs, G, c->sgs_twz.plan, c->sgs_twz.d);
-    c->launches += 3;
+    stress(F, c->mlp_tau);
   } else {
-  k_sgs_xpass1<<<gx, 128, sx11, c->stream>>>(c->sgs, G, c->sgs_twx.plan, c->sgs_twx.d, c->sgs_delta2, s2);
-  k_sgs_zfilt<KB><<<gz4, 256, sz, c->stream>>>(c->sgs, G, c->sgs_twz.plan, c->sgs_twz.d);
-  k_sgs_xpass2<<<gx, 128, sx11, c->stream>>>(c->sgs, G, c->sgs_twx.plan, c->sgs_twx.d, c->sgs_delta2);
-  k_sgs_coef<<<dim3((g.nx + 127) / 128, g.nyp), 128, 0, c->stream>>>(c->sgs, G, c->les_cs, c->les_ineg);
-  k_sgs_tau_x<<<gx, 128, sx3, c->stream>>>(c->sgs, G, c->sgs_twx.plan, c->sgs_twx.d, c->sgs_delta2, c->prm.re,
-                                           c->les_ineg, nullptr);
-  k_sgs_zfwd<KB><<<gz, 256, sz, c->stream>>>(c->sgs, G, c->sgs_twz.plan, c->sgs_twz.d);
-  c->launches += 7;
+    const double* s2 = nullptr;
+    if (c->iles == 3 && c->hpf_dyn) {
+      // dynamic HPF (bla/les.f:968-1383): first the strain of the secondary
+      // filtered field in physical space (test-filtered below in place of S),
+      // then u of the state with the strain of the primary filtered field
+      zinv(c->sgs, c->les_gu2, nullptr, 0, nullptr);
+      xinv9(c->hpf_s2, 3);
+      s2 = c->hpf_s2;
+      state_zinv(c->sgs, 0, c->les_gu);
+    } else if (c->iles == 3) {
+      // HPF model, fixed constant: the strain of the high-pass filtered fields
+      // (bla/les.f:404-450, 883-966)
+      zinv(c->sgs, c->les_gu, nullptr, 0, nullptr);
+    } else {
+      state_zinv(c->sgs, 0, nullptr);
+    }
+    coefficient(c->sgs, s2);
+    stress(c->sgs, nullptr);
   }
   // sigma on Chebyshev coefficients of tau (sgs_stress.f), back to physical y
   const size_t fld = (size_t)g.nyp * g.NP;
