@@ -9,8 +9,11 @@
 // small-radix Stockham passes (fft.cuh): the FP64 transforms were bound by
 // shared-memory bandwidth (80 % of its peak in the x pass at 192x129x160, FP64
 // pipe 21 %).  The buffer holds element (k1, n2) of column b at
-// k1 SR + n2 C + b with SR = C (mod 8): eight neighbouring items of either
-// pass touch eight different 16-byte bank groups.
+// k1 SR + n2 CS + b.  Eight neighbouring items of either pass touch eight
+// different 16-byte bank groups, in either order of the items:
+//   columns fastest (the z and Chebyshev transforms, whose columns are
+//   neighbours in memory): CS = C, SR = C (mod 8)
+//   elements fastest (NF; the x transforms, whose elements are): CS and SR odd
 //
 // Lengths are compile-time; R1 is a multiple of 3 for the 3/2-padded lengths,
 // so that the zero band is whole blocks of pass A's input (the middle third of
@@ -150,16 +153,20 @@ constexpr int f2_r1(int n) {
   return best;
 }
 
-template <int N, int C>
+template <int N, int C, bool NF = false>
 struct F2 {
   static constexpr int R1 = f2_r1(N), R2 = R1 ? N / (R1 ? R1 : 1) : 0;
   static_assert(R1 > 0, "no two-pass split of this length");
-  static constexpr int pad = ((C - R2 * C) % 8 + 8) % 8;
-  static constexpr int SR = R2 * C + pad;              // stride of k1
+  static constexpr int CS = NF ? (C | 1) : C;           // stride of n2
+  static constexpr int pad = NF ? (R2 * CS + 1) % 2 : ((C - R2 * C) % 8 + 8) % 8;
+  static constexpr int SR = R2 * CS + pad;              // stride of k1
   static constexpr int size = R1 * SR;                 // exchange buffer, elements
   static constexpr int items_a = R2 * C, items_b = R1 * C;
   static constexpr int items = items_a > items_b ? items_a : items_b;
-  static SB_HD __forceinline__ int at(int k1, int n2, int b) { return k1 * SR + n2 * C + b; }
+  static SB_HD __forceinline__ int at(int k1, int n2, int b) { return k1 * SR + n2 * CS + b; }
+  // item t of R elements by BC columns: its element and column
+  static SB_HD __forceinline__ int elem(int t, int R, int BC) { return NF ? t % R : t / BC; }
+  static SB_HD __forceinline__ int column(int t, int R, int BC) { return NF ? t / R : t % BC; }
 };
 
 // v[k] *= w^k, w = exp(S 2 pi i e / N), k < R, from the table tw[m] =
@@ -192,10 +199,10 @@ __device__ __forceinline__ void f2_twiddle(double2 (&v)[R], const double2* __res
 // -- with ZM the last third, n >= 2 N / 3, the others being n < N / 3 -- so
 // that a load needs no branch on n and a thread's loads go out together.  BC:
 // columns transformed (items t < R2 BC), C the buffer's.
-template <int N, int C, int BC, int S, bool ZM, class Ld>
+template <int N, int C, int BC, int S, bool ZM, bool NF = false, class Ld>
 __device__ __forceinline__ void f2_pass_a(Ld ld, double2* __restrict__ E, const double2* __restrict__ tw, int t) {
-  typedef F2<N, C> P;
-  const int n2 = t / BC, b = t - n2 * BC;
+  typedef F2<N, C, NF> P;
+  const int n2 = P::elem(t, P::R2, BC), b = P::column(t, P::R2, BC);
   double2 v[P::R1];
 #pragma unroll
   for (int n1 = 0; n1 < P::R1; ++n1)
@@ -208,10 +215,10 @@ __device__ __forceinline__ void f2_pass_a(Ld ld, double2* __restrict__ E, const 
 
 // Pass B of item t (< R1 BC): st(k, k1, k2, b, value) receives output
 // k = k1 + R1 k2.
-template <int N, int C, int BC, int S, class St>
+template <int N, int C, int BC, int S, bool NF = false, class St>
 __device__ __forceinline__ void f2_pass_b(St st, const double2* E, int t) {
-  typedef F2<N, C> P;
-  const int k1 = t / BC, b = t - k1 * BC;
+  typedef F2<N, C, NF> P;
+  const int k1 = P::elem(t, P::R1, BC), b = P::column(t, P::R1, BC);
   double2 v[P::R2];
 #pragma unroll
   for (int n2 = 0; n2 < P::R2; ++n2) v[n2] = E[P::at(k1, n2, b)];
@@ -226,11 +233,11 @@ __device__ __forceinline__ void f2_pass_b(St st, const double2* E, int t) {
 // ld); pass B, item q < R2, reads column q (DFT of R1): outputs k = q + R2 m.
 // col(b): the buffer column of transform b.  DROP: the middle third of m (the
 // dropped band of a forward transform) is neither computed nor stored.
-template <int N, int C, int BC, int S, class Ld, class Col>
+template <int N, int C, int BC, int S, bool NF, class Ld, class Col>
 __device__ __forceinline__ void f2_row_a(Ld ld, Col col, double2* E, const double2* __restrict__ tw,
                                          int t) {
-  typedef F2<N, C> P;
-  const int k1 = t / BC, b = t - k1 * BC;
+  typedef F2<N, C, NF> P;
+  const int k1 = P::elem(t, P::R1, BC), b = P::column(t, P::R1, BC);
   double2 v[P::R2];
 #pragma unroll
   for (int k2 = 0; k2 < P::R2; ++k2) v[k2] = ld(k1, k2, b);
@@ -239,19 +246,19 @@ __device__ __forceinline__ void f2_row_a(Ld ld, Col col, double2* E, const doubl
 #pragma unroll
   for (int k2 = 0; k2 < P::R2; ++k2) E[P::at(k1, k2, col(b))] = v[k2];
 }
-template <int N, int C, int BC, int S, class Col>
+template <int N, int C, int BC, int S, bool NF = false, class Col>
 __device__ __forceinline__ void f2_back_a(Col col, double2* E, const double2* __restrict__ tw, int t) {
-  f2_row_a<N, C, BC, S>([&](int k1, int k2, int b) { return E[F2<N, C>::at(k1, k2, col(b))]; }, col, E, tw, t);
+  f2_row_a<N, C, BC, S, NF>([&](int k1, int k2, int b) { return E[F2<N, C, NF>::at(k1, k2, col(b))]; }, col, E, tw, t);
 }
 template <int N, int C, int BC, int S, class Ld>
 __device__ __forceinline__ void f2_fwd_a(Ld ld, double2* __restrict__ E, const double2* __restrict__ tw, int t) {
-  f2_row_a<N, C, BC, S>([&](int k1, int k2, int b) { return ld(k1 + F2<N, C>::R1 * k2, b); }, [](int b) { return b; },
+  f2_row_a<N, C, BC, S, false>([&](int k1, int k2, int b) { return ld(k1 + F2<N, C>::R1 * k2, b); }, [](int b) { return b; },
                         E, tw, t);
 }
-template <int N, int C, int BC, int S, bool DROP, class St, class Col>
+template <int N, int C, int BC, int S, bool DROP, bool NF = false, class St, class Col>
 __device__ __forceinline__ void f2_back_b(St st, Col col, const double2* E, int t) {
-  typedef F2<N, C> P;
-  const int q = t / BC, b = t - q * BC;
+  typedef F2<N, C, NF> P;
+  const int q = P::elem(t, P::R2, BC), b = P::column(t, P::R2, BC);
   double2 v[P::R1];
 #pragma unroll
   for (int m = 0; m < P::R1; ++m) v[m] = E[P::at(m, q, col(b))];

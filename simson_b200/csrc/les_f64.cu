@@ -60,7 +60,7 @@ bool lf_xpass1(cudaStream_t s, const SgsBufs& B, const SgsGrid& G, const double2
   switch (G.nx) {
 #define SB_CASE(n) \
   case n:          \
-    lf_launch(k_sgs_xpass1_2<n>, grid, LF_XT, F2<n, 11>::size * 16, s, B, G, tw, delta2, s2); \
+    lf_launch(k_sgs_xpass1_2<n>, grid, LF_XT, F2<n, 11, true>::size * 16, s, B, G, tw, delta2, s2); \
     return true;
     SB_LF_LENGTHS(SB_CASE)
 #undef SB_CASE
@@ -73,7 +73,7 @@ bool lf_xpass2(cudaStream_t s, const SgsBufs& B, const SgsGrid& G, const double2
   switch (G.nx) {
 #define SB_CASE(n) \
   case n:          \
-    lf_launch(k_sgs_xpass2_2<n>, grid, LF_XT, F2<n, 11>::size * 16, s, B, G, tw, delta2); \
+    lf_launch(k_sgs_xpass2_2<n>, grid, LF_XT, F2<n, 11, true>::size * 16, s, B, G, tw, delta2); \
     return true;
     SB_LF_LENGTHS(SB_CASE)
 #undef SB_CASE
@@ -86,7 +86,7 @@ bool lf_xinv9(cudaStream_t s, const SgsBufs& B, const SgsGrid& G, const double2*
   switch (G.nx) {
 #define SB_CASE(n) \
   case n:          \
-    lf_launch(k_sgs_xinv9_2<n>, grid, LF_XT, F2<n, 5>::size * 16, s, B, G, tw, out, f0); \
+    lf_launch(k_sgs_xinv9_2<n>, grid, LF_XT, F2<n, 5, true>::size * 16, s, B, G, tw, out, f0); \
     return true;
     SB_LF_LENGTHS(SB_CASE)
 #undef SB_CASE
@@ -100,7 +100,7 @@ bool lf_tau_x(cudaStream_t s, const SgsBufs& B, const SgsGrid& G, const double2*
   switch (G.nx) {
 #define SB_CASE(n) \
   case n:          \
-    lf_launch(k_sgs_tau_x2<n>, grid, LF_XT, F2<n, 3>::size * 16, s, B, G, tw, delta2, re, ineg, tau_phys); \
+    lf_launch(k_sgs_tau_x2<n>, grid, LF_XT, F2<n, 3, true>::size * 16, s, B, G, tw, delta2, re, ineg, tau_phys); \
     return true;
     SB_LF_LENGTHS(SB_CASE)
 #undef SB_CASE

@@ -178,14 +178,14 @@ __device__ __forceinline__ double2 lf_pair(const double2* __restrict__ a, size_t
 template <int N, int C, int BC, int NF>
 __device__ __forceinline__ void lf_xinv(const double2* __restrict__ src, size_t fs, int nk, double2* E,
                                         const double2* __restrict__ tw, int t, int nt) {
-  typedef F2<N, C> P;
+  typedef F2<N, C, true> P;
   for (int i = t; i < P::R2 * BC; i += nt)
-    f2_pass_a<N, C, BC, 1, false>(
+    f2_pass_a<N, C, BC, 1, false, true>(
         [&](int k, int c, bool) { return lf_pair<NF>(src + (size_t)(2 * c) * fs, fs, c, k, N, nk); },
         E, tw, i);
   __syncthreads();
   for (int i = t; i < P::R1 * BC; i += nt)
-    f2_pass_b<N, C, BC, 1>([&](int, int k1, int k2, int b, double2 v) { E[P::at(k1, k2, b)] = v; }, E, i);
+    f2_pass_b<N, C, BC, 1, true>([&](int, int k1, int k2, int b, double2 v) { E[P::at(k1, k2, b)] = v; }, E, i);
   __syncthreads();
 }
 
@@ -194,12 +194,12 @@ __device__ __forceinline__ void lf_xinv(const double2* __restrict__ src, size_t 
 template <int N, int C, int BC, int NF>
 __device__ __forceinline__ void lf_xfwd(double2* __restrict__ dst, size_t fs, int nk, double2* E,
                                         const double2* __restrict__ tw, int t, int nt) {
-  typedef F2<N, C> P;
+  typedef F2<N, C, true> P;
   auto col = [](int b) { return b; };
-  for (int i = t; i < P::R1 * BC; i += nt) f2_back_a<N, C, BC, -1>(col, E, tw, i);
+  for (int i = t; i < P::R1 * BC; i += nt) f2_back_a<N, C, BC, -1, true>(col, E, tw, i);
   __syncthreads();
   for (int i = t; i < P::R2 * BC; i += nt)
-    f2_back_b<N, C, BC, -1, false>([&](int, int m, int q, int b, double2 v) { E[P::at(m, q, b)] = v; }, col, E, i);
+    f2_back_b<N, C, BC, -1, false, true>([&](int, int m, int q, int b, double2 v) { E[P::at(m, q, b)] = v; }, col, E, i);
   __syncthreads();
   for (int i = t; i < nk * BC; i += nt) {
     const int c = i / nk, k = i - c * nk, kk = k == 0 ? 0 : N - k;
@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(LF_XT) k_sgs_xpass1_2(SgsBufs B, SgsGrid G, co
                                                         const double* __restrict__ delta2,
                                                         const double* __restrict__ s2) {
   constexpr int C = 11;
-  typedef F2<N, C> P;
+  typedef F2<N, C, true> P;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double2* E = reinterpret_cast<double2*>(smem_raw);
   const int m = blockIdx.x, y = blockIdx.y, t = threadIdx.x;
@@ -267,7 +267,7 @@ template <int N>
 __global__ void __launch_bounds__(LF_XT) k_sgs_xpass2_2(SgsBufs B, SgsGrid G, const double2* __restrict__ tw,
                                                         const double* __restrict__ delta2) {
   constexpr int C = 11;
-  typedef F2<N, C> P;
+  typedef F2<N, C, true> P;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double2* E = reinterpret_cast<double2*>(smem_raw);
   const int m = blockIdx.x, y = blockIdx.y, t = threadIdx.x;
@@ -296,7 +296,7 @@ template <int N>
 __global__ void __launch_bounds__(LF_XT) k_sgs_xinv9_2(SgsBufs B, SgsGrid G, const double2* __restrict__ tw,
                                                        double* __restrict__ out, int f0) {
   constexpr int C = 5;
-  typedef F2<N, C> P;
+  typedef F2<N, C, true> P;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double2* E = reinterpret_cast<double2*>(smem_raw);
   const int m = blockIdx.x, y = blockIdx.y, t = threadIdx.x;
@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(LF_XT) k_sgs_tau_x2(SgsBufs B, SgsGrid G, cons
                                                       const double* __restrict__ delta2, double re, int ineg,
                                                       const double* __restrict__ tau_phys) {
   constexpr int C = 3;
-  typedef F2<N, C> P;
+  typedef F2<N, C, true> P;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double2* E = reinterpret_cast<double2*>(smem_raw);
   const int m = blockIdx.x, y = blockIdx.y, t = threadIdx.x;

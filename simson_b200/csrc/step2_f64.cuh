@@ -9,7 +9,13 @@
 //   k_zfwd2   eight kx columns
 //   k_xpass_p2  two z rows, six inverse and four forward columns
 // Three resident passes over shared memory per direction and column instead
-// of six.
+// of six.  At 384x193x384 against the Stockham kernels: z inverse 0.96 -> 0.63
+// ms, x pass 1.92 -> 1.49, z forward 0.51 -> 0.30 (moving 2.1, 3.1 and 1.5 GB;
+// 192x129x160: 0.13 -> 0.09, 0.35 -> 0.20, 0.06 -> 0.04).  Bound by the shared
+// memory and L1 traffic of the passes (x pass) and by HBM (z transforms).
+// The x passes' work items run along a row, as the rows do in memory; with
+// the columns fastest, as in the z transforms, the x pass took 1.97 ms: a warp's
+// load touched eleven rows.
 #pragma once
 #include "fft2.cuh"
 #include "layout.cuh"
@@ -132,7 +138,7 @@ __global__ void __launch_bounds__(f2_threads(F2<N, 3 * F2_RB>::items), f2_minb(f
              const double* __restrict__ dyi, double dxi, double dzi, double rot,
              unsigned long long* __restrict__ cfl_bits, Fringe fr) {
   constexpr int C = 3 * F2_RB, NT = f2_threads(F2<N, C>::items);
-  typedef F2<N, C> P;
+  typedef F2<N, C, true> P;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double2* E = reinterpret_cast<double2*>(smem_raw);
   const int y = g.y0 + blockIdx.y, m0 = blockIdx.x * F2_RB;
@@ -140,7 +146,7 @@ __global__ void __launch_bounds__(f2_threads(F2<N, 3 * F2_RB>::items), f2_minb(f
   const size_t row0 = ((size_t)y * g.nzp + m0) * g.nx2;
   const int t = threadIdx.x;
   if (t < P::items_a) {
-    f2_pass_a<N, C, C, 1, true>(
+    f2_pass_a<N, C, C, 1, true, true>(
         [&](int k, int c, bool high) {
           // (a row beyond the plane reads the last one; nothing of it is kept)
           const int q = c % 3, r = m0 + c / 3 < g.nzp ? c / 3 : 0;
@@ -152,39 +158,39 @@ __global__ void __launch_bounds__(f2_threads(F2<N, 3 * F2_RB>::items), f2_minb(f
   __syncthreads();
   // physical values back to their own row of the buffer: x = k1 + R1 k2 at (k1, k2)
   if (t < P::items_b)
-    f2_pass_b<N, C, C, 1>([&](int, int k1, int k2, int b, double2 v) { E[P::at(k1, k2, b)] = v; }, E, t);
+    f2_pass_b<N, C, C, 1, true>([&](int, int k1, int k2, int b, double2 v) { E[P::at(k1, k2, b)] = v; }, E, t);
   __syncthreads();
-  // products: row r of a point reads columns 3 r .. 3 r + 2 and leaves H1 + i H2
-  // in 3 r; row 0 leaves both rows' H3 in column 1
+  // products of both rows of a point: H1 + i H2 of row r over column 3 r, the
+  // two H3 over column 1
   const double r2 = 2.0 * rot, cy = dyi[y];
   double cmax = 0.0;
-  for (int t0 = 0; t0 < N * F2_RB; t0 += NT) {
-    const int i = t0 + t;
-    const bool in = i < N * F2_RB;
-    const int r = i & 1, pt = in ? i >> 1 : 0, k1 = pt / P::R2, k2 = pt - k1 * P::R2;
-    double2* e = E + P::at(k1, k2, 3 * r);
-    const double2 z0 = e[0], z1 = e[1], z2 = e[2];
-    const double u = z0.x, v = z0.y, w = z1.x, ox = z1.y, oy = z2.x, oz = z2.y;
-    double h1 = v * (oz + r2) - w * oy;
-    double h2 = w * ox - u * (oz + r2);
-    double h3 = u * oy - v * ox;
-    if (fr.lam != nullptr) fringe_apply<double>(fr, k1 + P::R1 * k2, y, g.nyp, N, u, v, w, 0.0, 0.0, h1, h2, h3);
-    const double h3o = __shfl_xor_sync(0xffffffffu, h3, 1);
-    if (in) {
-      e[0] = double2{h1, h2};
-      if (r == 0) e[1] = double2{h3, h3o};
+  for (int pt = t; pt < N; pt += NT) {
+    const int k1 = pt / P::R2, k2 = pt - k1 * P::R2;
+    double2* e = E + P::at(k1, k2, 0);
+    double h3r[F2_RB];
+#pragma unroll
+    for (int r = 0; r < F2_RB; ++r) {
+      const double2 z0 = e[3 * r], z1 = e[3 * r + 1], z2 = e[3 * r + 2];
+      const double u = z0.x, v = z0.y, w = z1.x, ox = z1.y, oy = z2.x, oz = z2.y;
+      double h1 = v * (oz + r2) - w * oy;
+      double h2 = w * ox - u * (oz + r2);
+      double h3 = u * oy - v * ox;
+      if (fr.lam != nullptr) fringe_apply<double>(fr, k1 + P::R1 * k2, y, g.nyp, N, u, v, w, 0.0, 0.0, h1, h2, h3);
+      e[3 * r] = double2{h1, h2};
+      h3r[r] = h3;
       if (m0 + r < g.nzp) cmax = fmax(cmax, fabs(u) * dxi + fabs(v) * cy + fabs(w) * dzi);
     }
+    e[1] = double2{h3r[0], h3r[1]};
   }
   __syncthreads();
   auto col = [](int b) { return b == 2 ? 3 : b; };
-  if (t < P::R1 * 3) f2_back_a<N, C, 3, -1>(col, E, tw, t);
+  if (t < P::R1 * 3) f2_back_a<N, C, 3, -1, true>(col, E, tw, t);
   __syncthreads();
   if (t < P::R2 * 3)
-    f2_back_b<N, C, 3, -1, true>([&](int, int m, int q, int b, double2 v) { E[P::at(m, q, b)] = v; }, col, E, t);
+    f2_back_b<N, C, 3, -1, true, true>([&](int, int m, int q, int b, double2 v) { E[P::at(m, q, b)] = v; }, col, E, t);
   __syncthreads();
   for (int i = t; i < g.nx2 * F2_RB; i += NT) {
-    const int k = i >> 1, r = i & 1;
+    const int r = i >= g.nx2, k = i - r * g.nx2;
     if (m0 + r >= g.nzp) continue;
     const int kk = k == 0 ? 0 : N - k;
     const double2* ek = E + P::at(k / P::R2, k % P::R2, 0);
@@ -213,7 +219,7 @@ template <int N>
 __global__ void __launch_bounds__(f2_threads(F2<N, 3 * F2_RB>::items), f2_minb(f2_threads(F2<N, 3 * F2_RB>::items)))
     k_xpass_p2(double2* zb, Dims g, const double2* __restrict__ tw, double rot, Fringe fr) {
   constexpr int C = 3 * F2_RB, NT = f2_threads(F2<N, C>::items);
-  typedef F2<N, C> P;
+  typedef F2<N, C, true> P;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double2* E = reinterpret_cast<double2*>(smem_raw);
   const int y = blockIdx.y, m0 = blockIdx.x * F2_RB;
@@ -221,7 +227,7 @@ __global__ void __launch_bounds__(f2_threads(F2<N, 3 * F2_RB>::items), f2_minb(f
   double2* row0 = zb + ((size_t)y * g.nzp + m0) * g.nx2;
   const int t = threadIdx.x;
   if (t < P::items_a) {
-    f2_pass_a<N, C, C, 1, true>(
+    f2_pass_a<N, C, C, 1, true, true>(
         [&](int k, int c, bool high) {
           const int q = c % 3, r = m0 + c / 3 < g.nzp ? c / 3 : 0;
           const double2* p0 = row0 + (size_t)(2 * q) * fstride + r * g.nx2;
@@ -231,11 +237,11 @@ __global__ void __launch_bounds__(f2_threads(F2<N, 3 * F2_RB>::items), f2_minb(f
   }
   __syncthreads();
   if (t < P::items_b)
-    f2_pass_b<N, C, C, 1>([&](int, int k1, int k2, int b, double2 v) { E[P::at(k1, k2, b)] = v; }, E, t);
+    f2_pass_b<N, C, C, 1, true>([&](int, int k1, int k2, int b, double2 v) { E[P::at(k1, k2, b)] = v; }, E, t);
   __syncthreads();
   const double r2 = 2.0 * rot;
   for (int i = t; i < N * F2_RB; i += NT) {
-    const int r = i & 1, pt = i >> 1, k1 = pt / P::R2, k2 = pt - k1 * P::R2;
+    const int r = i / N, pt = i - r * N, k1 = pt / P::R2, k2 = pt - k1 * P::R2;
     double2* e = E + P::at(k1, k2, 3 * r);
     const double2 z0 = e[0], z1 = e[1], z2 = e[2];
     const double u = z0.x, v = z0.y, w = z1.x, ox = z1.y, oy = z2.x, oz = z2.y;
@@ -248,13 +254,13 @@ __global__ void __launch_bounds__(f2_threads(F2<N, 3 * F2_RB>::items), f2_minb(f
   }
   __syncthreads();
   auto col = [](int b) { return b < 2 ? b : b + 1; };
-  if (t < P::R1 * 4) f2_back_a<N, C, 4, -1>(col, E, tw, t);
+  if (t < P::R1 * 4) f2_back_a<N, C, 4, -1, true>(col, E, tw, t);
   __syncthreads();
   if (t < P::R2 * 4)
-    f2_back_b<N, C, 4, -1, true>([&](int, int m, int q, int b, double2 v) { E[P::at(m, q, b)] = v; }, col, E, t);
+    f2_back_b<N, C, 4, -1, true, true>([&](int, int m, int q, int b, double2 v) { E[P::at(m, q, b)] = v; }, col, E, t);
   __syncthreads();
   for (int i = t; i < g.nx2 * F2_RB; i += NT) {
-    const int k = i >> 1, r = i & 1;
+    const int r = i >= g.nx2, k = i - r * g.nx2;
     if (m0 + r >= g.nzp) continue;
     const int kk = k == 0 ? 0 : N - k;
     const double2* ek = E + P::at(k / P::R2, k % P::R2, 3 * r);

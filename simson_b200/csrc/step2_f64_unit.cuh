@@ -12,9 +12,9 @@ template <class K>
 static void f2_smem(K kernel, int bytes) {
   cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
-template <int N, int C>
+template <int N, int C, bool NF = false>
 constexpr int f2_bytes() {
-  return F2<N, C>::size * (int)sizeof(double2);
+  return F2<N, C, NF>::size * (int)sizeof(double2);
 }
 
 bool SB_F2_CAT(f2_zinv_, SB_F2_UNIT)(cudaStream_t s, const double2* st, const float2* stf, double2* zb, const Dims& g,
@@ -63,7 +63,7 @@ bool SB_F2_CAT(f2_xpass_, SB_F2_UNIT)(cudaStream_t s, const double2* zb, double2
   switch (g.nxp) {
 #define SB_CASE(n)                                                                         \
   case n: {                                                                                \
-    constexpr int nt = f2_threads(F2<n, 3 * F2_RB>::items), sm = f2_bytes<n, 3 * F2_RB>(); \
+    constexpr int nt = f2_threads(F2<n, 3 * F2_RB>::items), sm = f2_bytes<n, 3 * F2_RB, true>(); \
     f2_smem(k_xpass2<n>, sm);                                                              \
     k_xpass2<n><<<grid, nt, sm, s>>>(zb, xb, g, tw, dyi, dxi, dzi, rot, cfl, fr);          \
     return true;                                                                           \
@@ -80,7 +80,7 @@ bool SB_F2_CAT(f2_xpass_p_, SB_F2_UNIT)(cudaStream_t s, double2* zb, const Dims&
   switch (g.nxp) {
 #define SB_CASE(n)                                                                         \
   case n: {                                                                                \
-    constexpr int nt = f2_threads(F2<n, 3 * F2_RB>::items), sm = f2_bytes<n, 3 * F2_RB>(); \
+    constexpr int nt = f2_threads(F2<n, 3 * F2_RB>::items), sm = f2_bytes<n, 3 * F2_RB, true>(); \
     f2_smem(k_xpass_p2<n>, sm);                                                            \
     k_xpass_p2<n><<<grid, nt, sm, s>>>(zb, g, tw, rot, fr);                                \
     return true;                                                                           \
