@@ -12,7 +12,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 LIB_DIR = os.path.join(HERE, "_lib")
 LIB = os.path.join(LIB_DIR, "libsimson_b200.so")
-UNITS = ["simson", "noalloc", "mixed", "pencil_chunk", "cheb_f64", "les_f64", "step2_f64"] + ["step2_f64_" + u for u in "abcd"]
+UNITS = ["simson", "noalloc", "mixed", "pencil_chunk", "cheb_f64", "les_f64", "xys_f64", "step2_f64"] + ["step2_f64_" + u for u in "abcd"]
 SOURCES = [os.path.join(HERE, "csrc", u + ".cu") for u in UNITS]
 # units built without fused multiply-add contraction: the host unit with the
 # kernels that keep the reference's rounding, and the allocation-free step 2

@@ -1740,27 +1740,35 @@ extern "C" int sgpu_xys_sample(sgpu_ctx* c, double dtn) {
   const size_t sx = 2 * (size_t)g.nx * XYS_NC * sizeof(double2);
   // the pressure entries when the pressure of this state has been computed
   const bool pres = c->press_valid && c->press;
-  xys_fields(c, pres ? c->press : nullptr);
-  const int nt = (g.nx + 31) / 32 * 32;
-  const dim3 gr(XYS_GROUPS, g.nyp);
   const double cw = dtn / (double)g.nz;
-  // the 384-thread instances (more registers per thread) whenever nx fits
-  if (pres && nt <= 384)
-    k_xys_acc<true, 384><<<gr, nt, sx, c->stream>>>(c->xys_spec, c->xys_part, c->xys_u, G, c->xys_twx.plan,
-                                                    c->xys_twx.d, cw);
-  else if (pres)
-    k_xys_acc<true><<<gr, nt, sx, c->stream>>>(c->xys_spec, c->xys_part, c->xys_u, G, c->xys_twx.plan, c->xys_twx.d,
-                                               cw);
-  else if (nt <= 384)
-    k_xys_acc<false, 384><<<gr, nt, sx, c->stream>>>(c->xys_spec, c->xys_part, c->xys_u, G, c->xys_twx.plan,
-                                                     c->xys_twx.d, cw);
-  else
-    k_xys_acc<false><<<gr, nt, sx, c->stream>>>(c->xys_spec, c->xys_part, c->xys_u, G, c->xys_twx.plan, c->xys_twx.d,
-                                                cw);
+  const double2* pr = pres ? c->press : nullptr;
+  const double* u = c->xys_u;  // u in physical space
+  if (xys_sums2(c->stream, c->st, c->mixed ? c->stf : nullptr, pr, c->xys_spec, c->xys_part, G, c->xys_twz.d,
+                c->xys_twx.d, c->alfa, c->beta, cw)) {
+    u = reinterpret_cast<const double*>(c->xys_spec);
+    c->launches += 2;
+  } else {
+    xys_fields(c, pr);
+    const int nt = (g.nx + 31) / 32 * 32;
+    const dim3 gr(XYS_GROUPS, g.nyp);
+    // the 384-thread instances (more registers per thread) whenever nx fits
+    if (pres && nt <= 384)
+      k_xys_acc<true, 384><<<gr, nt, sx, c->stream>>>(c->xys_spec, c->xys_part, c->xys_u, G, c->xys_twx.plan,
+                                                      c->xys_twx.d, cw);
+    else if (pres)
+      k_xys_acc<true><<<gr, nt, sx, c->stream>>>(c->xys_spec, c->xys_part, c->xys_u, G, c->xys_twx.plan, c->xys_twx.d,
+                                                 cw);
+    else if (nt <= 384)
+      k_xys_acc<false, 384><<<gr, nt, sx, c->stream>>>(c->xys_spec, c->xys_part, c->xys_u, G, c->xys_twx.plan,
+                                                       c->xys_twx.d, cw);
+    else
+      k_xys_acc<false><<<gr, nt, sx, c->stream>>>(c->xys_spec, c->xys_part, c->xys_u, G, c->xys_twx.plan,
+                                                  c->xys_twx.d, cw);
+  }
   const size_t plane = (size_t)g.nyp * g.nx;
   const int nb = (int)((plane + 255) / 256);
-  k_xys_add<<<nb, 256, 0, c->stream>>>(c->xys_part, c->xys, G, pres ? XYS_NACC_P : XYS_NACC);
-  k_xys_minmax<<<nb, 256, 0, c->stream>>>(c->xys_u, c->xys, G);
+  k_xys_add<<<dim3(nb, pres ? XYS_NACC_P : XYS_NACC), 256, 0, c->stream>>>(c->xys_part, c->xys, G);
+  k_xys_minmax<<<(unsigned)((plane + 31) / 32), 32 * XYS_MZ, 0, c->stream>>>(u, c->xys, G);
   c->launches += 3;
   c->xys_sumw += dtn;
   CK(cudaGetLastError());

@@ -30,8 +30,10 @@
 //                 accumulated in registers by the thread that owns its x;
 //                 the group's sums and the physical u rows written out
 //   k_xys_add     per (y, x): the groups' sums added to xys in group order
-//   k_xys_minmax  per (y, x): <u>_z in z order, then the running min / max
-//                 of u - <u>_z (boxxys.f:991-1035)
+//   k_xys_minmax  per (y, x): <u>_z, then the running min / max of u - <u>_z
+//                 (boxxys.f:991-1035)
+// Lengths with two-pass transforms take xys_f64.cuh's kernels in the place of
+// the first two.
 //
 // FP64 arithmetic whatever the state storage.  Device layout of xys:
 // [s][y][x] (the reference's xys(x, y, s) with leading dimensions nx, nyp).
@@ -105,10 +107,85 @@ __global__ void k_xys_zinv(const V* __restrict__ st, const double2* __restrict__
   }
 }
 
+// The moments of one point: q = u v w, omega x y z, du_i/dx_j (i-major), p; c =
+// dtn / nz, the weight of one point (boxxys.f:556, nfzsym = 0).
+template <bool PRES>
+__device__ __forceinline__ void xys_accumulate(const double (&q)[16], double c,
+                                               double (&acc)[PRES ? XYS_NACC_P : XYS_NACC]) {
+  const double u = q[0], v = q[1], w = q[2];
+  const double* om = q + 3;
+  const double* du = q + 6;  // du[3 i + j] = du_i / dx_j
+  const double uu = u * u, vv = v * v, ww = w * w;
+  acc[0] += u * c;
+  acc[1] += v * c;
+  acc[2] += w * c;
+  acc[3] += uu * c;
+  acc[4] += vv * c;
+  acc[5] += ww * c;
+  acc[6] += om[0] * c;
+  acc[7] += om[1] * c;
+  acc[8] += om[2] * c;
+  acc[9] += om[0] * om[0] * c;
+  acc[10] += om[1] * om[1] * c;
+  acc[11] += om[2] * om[2] * c;
+  acc[12] += u * v * c;
+  acc[13] += u * w * c;
+  acc[14] += v * w * c;
+  // dissipation tensor re eps_ij = du_i/dx_k du_j/dx_k (boxxys.f:849-891)
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+    acc[15 + i] += (du[3 * i] * du[3 * i] + du[3 * i + 1] * du[3 * i + 1] + du[3 * i + 2] * du[3 * i + 2]) * c;
+  acc[18] += (du[0] * du[3] + du[1] * du[4] + du[2] * du[5]) * c;
+  acc[19] += (du[0] * du[6] + du[1] * du[7] + du[2] * du[8]) * c;
+  acc[20] += (du[3] * du[6] + du[4] * du[7] + du[5] * du[8]) * c;
+  // strain rate (boxxys.f:1037-1090)
+  const double s1 = du[0], s2 = .5 * (du[3] + du[1]), s3 = .5 * (du[6] + du[2]);
+  const double s4 = du[4], s5 = .5 * (du[5] + du[7]), s6 = du[8];
+  acc[21] += (s1 * s1 + s4 * s4 + s6 * s6 + 2. * (s2 * s2 + s3 * s3 + s5 * s5)) * c;
+  acc[22] += s1 * c;
+  acc[23] += s2 * c;
+  acc[24] += s3 * c;
+  acc[25] += s4 * c;
+  acc[26] += s5 * c;
+  acc[27] += s6 * c;
+  // third and fourth moments (boxxys.f:1276-1380)
+  acc[28] += uu * u * c;
+  acc[29] += vv * v * c;
+  acc[30] += ww * w * c;
+  acc[31] += uu * v * c;
+  acc[32] += uu * w * c;
+  acc[33] += vv * u * c;
+  acc[34] += vv * w * c;
+  acc[35] += ww * u * c;
+  acc[36] += ww * v * c;
+  acc[37] += u * v * w * c;
+  acc[38] += uu * uu * c;
+  acc[39] += vv * vv * c;
+  acc[40] += ww * ww * c;
+  if constexpr (PRES) {
+    const double p = q[15];
+    acc[41] += p * c;
+    acc[42] += p * p * c;
+    acc[43] += u * p * c;
+    acc[44] += v * p * c;
+    acc[45] += w * p * c;
+    acc[46] += p * du[0] * c;  // p ux
+    acc[47] += p * du[4] * c;  // p vy
+    acc[48] += p * du[8] * c;  // p wz
+    acc[49] += p * du[1] * c;  // p uy
+    acc[50] += p * du[5] * c;  // p vz
+    acc[51] += p * du[6] * c;  // p wx
+    acc[52] += p * du[2] * c;  // p uz
+    acc[53] += p * du[3] * c;  // p vx
+    acc[54] += p * du[7] * c;  // p wy
+    acc[55] += p * p * p * c;
+    acc[56] += p * p * (p * p) * c;
+  }
+}
+
 // blockDim.x >= nx (nx <= MAXT <= 512); thread j owns x = j.  part: [XYS_GROUPS][XYS_NACC_P][nyp][nx];
 // PRES: the pressure entries too (field 15 holds p).
-// uphys: [nyp][nz][nx].  c = dtn / nz, the weight of one point
-// (boxxys.f:556, nfzsym = 0).
+// uphys: [nyp][nz][nx].
 // MAXT: the block size the register budget is sized for.  The accumulators
 // stay in registers across the z rows: at 512 threads (128 registers) 512
 // bytes of them spill (240 without the pressure entries), at 384 threads
@@ -147,76 +224,8 @@ __global__ void __launch_bounds__(MAXT) k_xys_acc(const double2* __restrict__ sp
         q[2 * cc] = z.x;
         q[2 * cc + 1] = z.y;
       }
-      const double u = q[0], v = q[1], w = q[2];
-      const double* om = q + 3;
-      const double* du = q + 6;  // du[3 i + j] = du_i / dx_j
-      uphys[((size_t)y * G.nz + m) * n + j] = u;
-      const double uu = u * u, vv = v * v, ww = w * w;
-      acc[0] += u * c;
-      acc[1] += v * c;
-      acc[2] += w * c;
-      acc[3] += uu * c;
-      acc[4] += vv * c;
-      acc[5] += ww * c;
-      acc[6] += om[0] * c;
-      acc[7] += om[1] * c;
-      acc[8] += om[2] * c;
-      acc[9] += om[0] * om[0] * c;
-      acc[10] += om[1] * om[1] * c;
-      acc[11] += om[2] * om[2] * c;
-      acc[12] += u * v * c;
-      acc[13] += u * w * c;
-      acc[14] += v * w * c;
-      // dissipation tensor re eps_ij = du_i/dx_k du_j/dx_k (boxxys.f:849-891)
-#pragma unroll
-      for (int i = 0; i < 3; ++i)
-        acc[15 + i] += (du[3 * i] * du[3 * i] + du[3 * i + 1] * du[3 * i + 1] + du[3 * i + 2] * du[3 * i + 2]) * c;
-      acc[18] += (du[0] * du[3] + du[1] * du[4] + du[2] * du[5]) * c;
-      acc[19] += (du[0] * du[6] + du[1] * du[7] + du[2] * du[8]) * c;
-      acc[20] += (du[3] * du[6] + du[4] * du[7] + du[5] * du[8]) * c;
-      // strain rate (boxxys.f:1037-1090)
-      const double s1 = du[0], s2 = .5 * (du[3] + du[1]), s3 = .5 * (du[6] + du[2]);
-      const double s4 = du[4], s5 = .5 * (du[5] + du[7]), s6 = du[8];
-      acc[21] += (s1 * s1 + s4 * s4 + s6 * s6 + 2. * (s2 * s2 + s3 * s3 + s5 * s5)) * c;
-      acc[22] += s1 * c;
-      acc[23] += s2 * c;
-      acc[24] += s3 * c;
-      acc[25] += s4 * c;
-      acc[26] += s5 * c;
-      acc[27] += s6 * c;
-      // third and fourth moments (boxxys.f:1276-1380)
-      acc[28] += uu * u * c;
-      acc[29] += vv * v * c;
-      acc[30] += ww * w * c;
-      acc[31] += uu * v * c;
-      acc[32] += uu * w * c;
-      acc[33] += vv * u * c;
-      acc[34] += vv * w * c;
-      acc[35] += ww * u * c;
-      acc[36] += ww * v * c;
-      acc[37] += u * v * w * c;
-      acc[38] += uu * uu * c;
-      acc[39] += vv * vv * c;
-      acc[40] += ww * ww * c;
-      if constexpr (PRES) {
-        const double p = q[15];
-        acc[41] += p * c;
-        acc[42] += p * p * c;
-        acc[43] += u * p * c;
-        acc[44] += v * p * c;
-        acc[45] += w * p * c;
-        acc[46] += p * du[0] * c;  // p ux
-        acc[47] += p * du[4] * c;  // p vy
-        acc[48] += p * du[8] * c;  // p wz
-        acc[49] += p * du[1] * c;  // p uy
-        acc[50] += p * du[5] * c;  // p vz
-        acc[51] += p * du[6] * c;  // p wx
-        acc[52] += p * du[2] * c;  // p uz
-        acc[53] += p * du[3] * c;  // p vx
-        acc[54] += p * du[7] * c;  // p wy
-        acc[55] += p * p * p * c;
-        acc[56] += p * p * (p * p) * c;
-      }
+      uphys[((size_t)y * G.nz + m) * n + j] = q[0];
+      xys_accumulate<PRES>(q, c, acc);
     }
     __syncthreads();
   }
@@ -228,31 +237,55 @@ __global__ void __launch_bounds__(MAXT) k_xys_acc(const double2* __restrict__ sp
   }
 }
 
-__global__ void k_xys_add(const double* __restrict__ part, double* __restrict__ xys, SgsGrid G, int nacc) {
+// one entry per blockIdx.y
+static __global__ void k_xys_add(const double* __restrict__ part, double* __restrict__ xys, SgsGrid G) {
   const size_t plane = (size_t)G.nyp * G.nx;
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= plane) return;
-  for (int k = 0; k < nacc; ++k) {
-    double s = 0.0;
-    for (int grp = 0; grp < XYS_GROUPS; ++grp) s += part[((size_t)grp * XYS_NACC_P + k) * plane + i];
-    xys[(size_t)(xys_entry(k) - 1) * plane + i] += s;
-  }
+  const int k = blockIdx.y;
+  double v[XYS_GROUPS], s = 0.0;
+#pragma unroll
+  for (int grp = 0; grp < XYS_GROUPS; ++grp) v[grp] = part[((size_t)grp * XYS_NACC_P + k) * plane + i];
+#pragma unroll
+  for (int grp = 0; grp < XYS_GROUPS; ++grp) s += v[grp];
+  xys[(size_t)(xys_entry(k) - 1) * plane + i] += s;
 }
 
-__global__ void k_xys_minmax(const double* __restrict__ uphys, double* __restrict__ xys, SgsGrid G) {
+// 32 points of the plane [y][x] per CTA (nx is a multiple of four, so a run of
+// 32 may cross into the next y), XYS_MZ groups of z rows
+constexpr int XYS_MZ = 8;
+static __global__ void __launch_bounds__(32 * XYS_MZ) k_xys_minmax(const double* __restrict__ uphys,
+                                                                   double* __restrict__ xys, SgsGrid G) {
+  __shared__ double sh[XYS_MZ][32], sx[XYS_MZ][32];
   const size_t plane = (size_t)G.nyp * G.nx;
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= plane) return;
-  const int y = (int)(i / G.nx), x = (int)(i - (size_t)y * G.nx);
+  const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5;
+  const size_t i = (size_t)blockIdx.x * 32 + lane;
+  const bool in = i < plane;
+  const int y = in ? (int)(i / G.nx) : 0, x = in ? (int)(i - (size_t)y * G.nx) : 0;
   const double* u = uphys + (size_t)y * G.nz * G.nx + x;
-  double ut = 0.0;
-  for (int m = 0; m < G.nz; ++m) ut = ut + u[(size_t)m * G.nx];
+  double ut = 0.0, lo = HUGE_VAL, hi = -HUGE_VAL;
+  for (int m = grp; m < G.nz; m += XYS_MZ) ut = ut + u[(size_t)m * G.nx];
+  sh[grp][lane] = ut;
+  __syncthreads();
+  ut = 0.0;
+#pragma unroll
+  for (int g = 0; g < XYS_MZ; ++g) ut = ut + sh[g][lane];
   ut = ut / (double)G.nz;
-  double umin = xys[(size_t)42 * plane + i], umax = xys[(size_t)43 * plane + i];
-  for (int m = 0; m < G.nz; ++m) {
+  __syncthreads();
+  for (int m = grp; m < G.nz; m += XYS_MZ) {
     const double d = u[(size_t)m * G.nx] - ut;
-    umax = fmax(umax, d);
-    umin = fmin(umin, d);
+    hi = fmax(hi, d);
+    lo = fmin(lo, d);
+  }
+  sh[grp][lane] = lo;
+  sx[grp][lane] = hi;
+  __syncthreads();
+  if (grp != 0 || !in) return;
+  double umin = xys[(size_t)42 * plane + i], umax = xys[(size_t)43 * plane + i];
+#pragma unroll
+  for (int g = 0; g < XYS_MZ; ++g) {
+    umin = fmin(umin, sh[g][lane]);
+    umax = fmax(umax, sx[g][lane]);
   }
   xys[(size_t)42 * plane + i] = umin;
   xys[(size_t)43 * plane + i] = umax;
@@ -267,7 +300,7 @@ __global__ void k_xys_minmax(const double* __restrict__ uphys, double* __restric
 // targets[6] = tau_ij = <u_i u_j> - <u_i> <u_j> (11 12 13 22 23 33): the
 // inputs and the output of the model of sgs_mlp.cuh, unscaled.  One CTA per
 // (Z, y), blockDim >= nx / f; reads the spectral fields of k_xys_zinv.
-__global__ void __launch_bounds__(512) k_box_sample(const double2* __restrict__ spec, SgsGrid G, FFTPlan plan,
+static __global__ void __launch_bounds__(512) k_box_sample(const double2* __restrict__ spec, SgsGrid G, FFTPlan plan,
                                                     const double2* __restrict__ tw, int f,
                                                     float* __restrict__ features, float* __restrict__ targets) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
