@@ -26,4 +26,8 @@ bool pencil_chunk(cudaStream_t s, const PencilBufs& B, const Dims& g, const doub
   return launch_pencil_chunk(s, B, g, alfa, beta, re, rk, cl, cv, rows, mean);
 }
 
+bool press_chunk(cudaStream_t s, const PressArgs& P, const Dims& g, const double* cv, const double2* rows) {
+  return launch_press_chunk(s, P, g, cv, rows);
+}
+
 }  // namespace sb

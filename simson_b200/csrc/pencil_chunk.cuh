@@ -36,6 +36,7 @@
 // 48x65x48 60 -> 12 us, 64x97x64 62 -> 23, 192x129x160 591 -> 178,
 // 384x193x384 1810 -> 1250.
 #pragma once
+#include "press.cuh"
 #include "step3.cuh"
 
 namespace sb {
@@ -217,12 +218,17 @@ __device__ __forceinline__ void pc_summary(const double (&f)[NC][R], const doubl
   }
 }
 
+struct PcClass {
+  double p, q, kp, kq;
+};
+
 // The walks of both parities (one warp: lane = (parity * 4 + column) * PC_TP +
 // pencil).  Leaves X in the u slots, Yp in the P slots and Yq in the N slot of
-// each chunk; the class's first unknown y and the sums go to the caller.  The
+// each chunk; the class's sums P + Q y of x (p, q) and of k^2 x (kp, kq; K),
+// which fix its first unknown y, go to the caller.  The
 // chains are FP64 latencies; the summaries of PC_WB chunks are read ahead.
 template <int NC, bool K>
-__device__ __forceinline__ void pc_walk(const PcArea& A, int G, int lane, double& y, double& sq, double& slope) {
+__device__ __forceinline__ PcClass pc_walk(const PcArea& A, int G, int lane) {
   typedef PcSum<NC, K> S;
   const int q = lane % PC_TP, col = (lane / PC_TP) & 3, par = lane / (4 * PC_TP);
   const bool own = col < NC;
@@ -294,9 +300,7 @@ __device__ __forceinline__ void pc_walk(const PcArea& A, int G, int lane, double
       for (int i = 0; i < PC_WB; ++i) b0[o + i * PC_TP + S::oN * PC_S] = yq[i];
     }
   }
-  y = -Sp / Sq;
-  sq = Sq;
-  slope = fma_(y, lq, lp);
+  return PcClass{Sp, Sq, lp, lq};
 }
 
 // x_j = P + PM X + N Y of the chunk's rows, in f
@@ -448,9 +452,8 @@ __device__ __forceinline__ void pc_mean(const MeanArgs& M, const Dims& g, double
     if (chunk) pc_summary<R, 4, false>(f, PM, N, A, t, (double)j0);
     __syncthreads();
     if (tid < 32) {
-      double y, sq, sl;
-      pc_walk<4, false>(A, G, tid, y, sq, sl);
-      ysm[tid] = y;
+      const PcClass w = pc_walk<4, false>(A, G, tid);
+      ysm[tid] = -w.p / w.q;
     }
     __syncthreads();
     pc_finish<R, 4, false>(f, PM, N, A, ysm, t, q);
@@ -731,10 +734,9 @@ __global__ void __launch_bounds__((PC_NT + 31) / 32 * 32, pc_minb(R))
     if (chunk) pc_summary<R, 4, false>(f, PM, N, A, t, dj0);
     __syncthreads();
     if (tid < 32) {
-      double y, sq, sl;
-      pc_walk<4, false>(A, G, tid, y, sq, sl);
-      ysm[tid] = y;
-      if (((tid / PC_TP) & 3) == 0) sqi[tid / (4 * PC_TP) * PC_TP + q] = 1.0 / sq;
+      const PcClass w = pc_walk<4, false>(A, G, tid);
+      ysm[tid] = -w.p / w.q;  // zero wall values
+      if (((tid / PC_TP) & 3) == 0) sqi[tid / (4 * PC_TP) * PC_TP + q] = 1.0 / w.q;
     }
     __syncthreads();
     pc_finish<R, 4, false>(f, PM, N, A, ysm, t, q);
@@ -771,8 +773,8 @@ __global__ void __launch_bounds__((PC_NT + 31) / 32 * 32, pc_minb(R))
     if (chunk) pc_summary<R, 3, true>(vv, PM, N, A, t, dj0);
     __syncthreads();
     if (tid < 32) {
-      double y, sq, sl;
-      pc_walk<3, true>(A, G, tid, y, sq, sl);
+      const PcClass w = pc_walk<3, true>(A, G, tid);
+      const double y = -w.p / w.q, sl = fma_(y, w.kq, w.kp);
       // dv/dy = 0 at the walls (linearbl.f:1020-1085): the class sum of k^2
       // v_k is the slope, which v_h takes out
       const int col = (tid / PC_TP) & 3, par = tid / (4 * PC_TP);
@@ -882,6 +884,147 @@ __global__ void __launch_bounds__((PC_NT + 31) / 32 * 32, pc_minb(R))
   }
 }
 
+// The pressure's pencils (press.cuh, k_press: the same system and Neumann data,
+// bla/linearp.f:77-158) but kx = kz = 0, chunked as above: f = D H2 + (i alpha
+// H1 + i beta H3), (D^2 - k^2) x = f with D x at the walls (the class sums of
+// k^2 x fix the first unknowns), p = x - E.  The thread-per-pencil kernel took
+// 0.58 ms at 192x129x160 for 0.25 GB, one wave of serial walks; this one
+// 0.095.
+template <int R, class VT>
+__global__ void __launch_bounds__((PC_NT + 31) / 32 * 32, pc_minb(R))
+    k_press_c(PressArgs P, const VT* __restrict__ V, Dims g, const double* __restrict__ CV,
+              const double2* __restrict__ rows, int G) {
+  extern __shared__ __align__(16) unsigned char pc_smem[];
+  __shared__ double ysm[2 * 4 * PC_TP];
+  __shared__ double wall[4 * PC_TP];  // D^2 v at y = +1, -1 of each pencil, real and imaginary
+  const int tid = threadIdx.x, nt = G * PC_TP;
+  const bool chunk = tid < nt;
+  const int q = tid % PC_TP, c = chunk ? tid / PC_TP : 0;
+  const int t = chunk ? tid : q;
+  const PcArea A{reinterpret_cast<double*>(pc_smem)};
+  double* cs = A.p + PC_AREA * PC_S + t;
+  const int n = g.nyp;
+  const size_t NP = g.NP;
+  const int p = blockIdx.x * PC_TP + q;
+  const int pc = min(p, g.NP - 1);
+  const int kx = pc % g.nx2, iz = pc / g.nx2;
+  const bool act = chunk && p < g.NP && iz != g.zodd && p != 0;
+  const double a = P.alfa[kx], be = P.beta[iz];
+  const double k2 = (pc == 0) ? 1.0 : a * a + be * be;
+  const int na = (g.nz / 2 + 1) * g.nx2;
+  const int pa = min(iz, g.nz - iz) * g.nx2 + kx;
+  const int j0 = c * R;
+  const double dj0 = (double)j0, w0 = 2.0 * dj0;
+  auto row_in = [&](int r) { return chunk && j0 + r < n; };
+  double f[2][R];
+  // D H2 by the suffix walk, D^2 v at the walls by the quadrature weights
+  {
+    double hx[R], hy[R], T[4] = {0.0, 0.0, 0.0, 0.0}, S[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      double2 h{0.0, 0.0}, d{0.0, 0.0};
+      if (row_in(r)) {
+        const int j = j0 + r;
+        const size_t o = (size_t)j * NP + pc;
+        h = P.CH2[o];
+        d = P.CD[o];
+        const VT v = V[o];
+        const double w1 = __ldg(&P.wd[j]), w2 = __ldg(&P.wd[n + j]);
+        S[0] = fma_((double)v.x, w1, S[0]);
+        S[1] = fma_((double)v.x, w2, S[1]);
+        S[2] = fma_((double)v.y, w1, S[2]);
+        S[3] = fma_((double)v.y, w2, S[3]);
+        cs[r * PC_NT] = CV[(size_t)j * na + pa];
+      } else if (chunk) {
+        cs[r * PC_NT] = 0.0;
+      }
+      hx[r] = h.x;
+      hy[r] = h.y;
+      f[0][r] = d.x;
+      f[1][r] = d.y;
+    }
+#pragma unroll
+    for (int r = R - 1; r >= 0; --r) {
+      const double w = w0 + (double)(2 * r);
+      T[r & 1] = fma_(w, hx[r], T[r & 1]);
+      T[2 + (r & 1)] = fma_(w, hy[r], T[2 + (r & 1)]);
+    }
+    if (chunk) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        A.at(i, t) = T[i];
+        A.at(4 + i, t) = S[i];
+      }
+    }
+    __syncthreads();
+    if (tid < 4 * PC_TP) {
+      pc_dwalk1(A, G, tid / PC_TP, q);
+    } else if (tid >= 32 - 4 * PC_TP && tid < 32) {
+      const int i = (tid - (32 - 4 * PC_TP)) / PC_TP;
+      double s = 0.0;
+      for (int cc = 0; cc < G; ++cc) s += A.at(4 + i, cc * PC_TP + q);
+      wall[i * PC_TP + q] = s;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) T[i] = A.at(i, t);
+#pragma unroll
+    for (int r = R - 1; r >= 0; --r) {
+      const double w = w0 + (double)(2 * r);
+      double dx = T[1 - (r & 1)], dy = T[3 - (r & 1)];
+      T[r & 1] = fma_(w, hx[r], T[r & 1]);
+      T[2 + (r & 1)] = fma_(w, hy[r], T[2 + (r & 1)]);
+      if (r == 0 && j0 == 0) {
+        dx *= 0.5;
+        dy *= 0.5;
+      }
+      f[0][r] = row_in(r) ? f[0][r] + dx : 0.0;
+      f[1][r] = row_in(r) ? f[1][r] + dy : 0.0;
+    }
+  }
+  __syncthreads();
+  if (chunk) {
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      A.at(4 * k + 0, t) = f[k][0];
+      A.at(4 * k + 1, t) = f[k][1];
+      A.at(4 * k + 2, t) = f[k][R - 2];
+      A.at(4 * k + 3, t) = f[k][R - 1];
+    }
+  }
+  __syncthreads();
+  double PM[R], N[R];
+  pc_local<R, 2>(f, PM, N, cs, rows + j0, 1.0 / k2, A, t, c > 0, c + 1 < G);
+  __syncthreads();
+  if (chunk) pc_summary<R, 2, true>(f, PM, N, A, t, dj0);
+  __syncthreads();
+  if (tid < 32) {
+    const PcClass w = pc_walk<2, true>(A, G, tid);
+    // D x at y = +1, -1: H2 + (D^2 v - k^2 v) / Re - dv/dt (linearp.f:77-150;
+    // v at the walls of the last step is zero)
+    const int col = (tid / PC_TP) & 1, par = tid / (4 * PC_TP);
+    double bc[2];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const size_t o = (e ? (size_t)(n - 1) * NP : 0) + pc;
+      const double2 h = P.PH2[o];
+      const double vw = col ? (double)V[o].y : (double)V[o].x;
+      bc[e] = (col ? h.y : h.x) * P.cn + (wall[(2 * col + e) * PC_TP + q] - k2 * vw) / P.re - vw * P.c4t;
+    }
+    const double b = par ? 0.5 * (bc[0] + bc[1]) : 0.5 * (bc[0] - bc[1]);
+    ysm[tid] = (b - w.kp) / w.kq;
+  }
+  __syncthreads();
+  pc_finish<R, 2, true>(f, PM, N, A, ysm, t, q);
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+    if (act && row_in(r)) {
+      const size_t o = (size_t)(j0 + r) * NP + pc;
+      const double2 ce = P.CE[o];
+      P.X[o] = double2{f[0][r] - ce.x, f[1][r] - ce.y};
+    }
+}
+
 // Rows per chunk for ny: 0 when ny is beyond the kernel's range
 inline int pencil_chunk_rows(int ny) {
 #ifdef SB_PC_R
@@ -911,6 +1054,34 @@ inline bool launch_pencil_chunk(cudaStream_t s, const PencilBufs& B, const Dims&
 #define SB_PC_CASE(RR)                                                         \
   case RR:                                                                     \
     pencil_chunk_n<RR>(s, B, g, alfa, beta, re, rk, CL, CV, rows, M); \
+    return true;
+    SB_PC_CASE(4) SB_PC_CASE(6) SB_PC_CASE(8) SB_PC_CASE(10)
+#undef SB_PC_CASE
+    default:
+      return false;
+  }
+}
+
+template <int R>
+inline void press_chunk_n(cudaStream_t s, const PressArgs& P, const Dims& g, const double* CV, const double2* rows) {
+  const int G = ((g.nyp + R - 1) / R + PC_WB - 1) / PC_WB * PC_WB, nt = G * PC_TP;
+  constexpr int smem = (PC_S * PC_AREA + PC_NT * R) * (int)sizeof(double);
+  const unsigned blocks = (unsigned)((g.NP + PC_TP - 1) / PC_TP);
+  if (P.Vf) {
+    cudaFuncSetAttribute(k_press_c<R, float2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    k_press_c<R, float2><<<blocks, (nt + 31) / 32 * 32, smem, s>>>(P, P.Vf, g, CV, rows, G);
+  } else {
+    cudaFuncSetAttribute(k_press_c<R, double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    k_press_c<R, double2><<<blocks, (nt + 31) / 32 * 32, smem, s>>>(P, P.V, g, CV, rows, G);
+  }
+}
+
+inline bool launch_press_chunk(cudaStream_t s, const PressArgs& P, const Dims& g, const double* CV,
+                               const double2* rows) {
+  switch (pencil_chunk_rows(g.nyp)) {
+#define SB_PC_CASE(RR)                        \
+  case RR:                                    \
+    press_chunk_n<RR>(s, P, g, CV, rows); \
     return true;
     SB_PC_CASE(4) SB_PC_CASE(6) SB_PC_CASE(8) SB_PC_CASE(10)
 #undef SB_PC_CASE

@@ -5,6 +5,7 @@
 #include <vector>
 
 #include "layout.cuh"
+#include "press.cuh"
 #include "step3.cuh"
 
 namespace sb {
@@ -20,5 +21,8 @@ void pencil_tau_coef(cudaStream_t s, double* out, const Dims& g, const double* a
 // in the same launch, or null
 bool pencil_chunk(cudaStream_t s, const PencilBufs& B, const Dims& g, const double* alfa, const double* beta,
                   double re, RKc rk, const double* cl, const double* cv, const double2* rows, const MeanArgs* mean);
+
+// the pressure's pencils but kx = kz = 0 (k_press_mean does that one)
+bool press_chunk(cudaStream_t s, const PressArgs& P, const Dims& g, const double* cv, const double2* rows);
 
 }  // namespace sb

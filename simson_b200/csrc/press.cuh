@@ -15,7 +15,9 @@
 //   step-2 z-forward (k_zfwd) of H1, H2, H3 and 2E into scratch fields
 //   k_press_div  i alpha H1 + i beta H3 (nonlinp.f:200-236)
 //   Chebyshev transforms of that, H2 and E (k_cheb)
-//   k_press      per pencil: the right-hand side, the Neumann data, the tau
+//   k_press_c (pencil_chunk.cuh) and k_press_mean, or, for ny beyond their
+//   range, k_press:
+//                per pencil: the right-hand side, the Neumann data, the tau
 //                solve of bla/crhsc.f, bla/setmac.f (neumann = 1) and
 //                bla/tridc.f, the mean mode by bla/icheb.f, minus E
 //   inverse Chebyshev transform of p (k_cheb)
@@ -36,7 +38,7 @@ namespace sb {
 // row: every read of it is done before the first barrier).
 // fr: the fringe forcing of a spatial run, which the reference's pressure
 // includes as well (bla/fringp.f, the forcing of bla/fring.f on H).
-__global__ void __launch_bounds__(256) k_xpass_p(double2* __restrict__ zb, Dims g, FFTPlan plan,
+static __global__ void __launch_bounds__(256) k_xpass_p(double2* __restrict__ zb, Dims g, FFTPlan plan,
                                                  const double2* __restrict__ tw, double rot, Fringe fr) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double2* bA = reinterpret_cast<double2*>(smem_raw);
@@ -92,7 +94,7 @@ __global__ void __launch_bounds__(256) k_xpass_p(double2* __restrict__ zb, Dims 
 
 // h[0] <- i alpha H1 + i beta H3 (h[0] = H1, h[2] = H3 on entry), every
 // stored mode of every plane (nonlinp.f:200-236, stored as linearp reads it)
-__global__ void k_press_div(double2* __restrict__ h, Dims g, const double* __restrict__ alfa,
+static __global__ void k_press_div(double2* __restrict__ h, Dims g, const double* __restrict__ alfa,
                             const double* __restrict__ beta) {
   const size_t fld = (size_t)g.nyp * g.NP;
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -159,7 +161,36 @@ __device__ __forceinline__ double2 vload(const PressArgs& A, size_t i) {
   return A.V[i];
 }
 
-__global__ void __launch_bounds__(128) k_press(PressArgs A, Dims g) {
+// kx = kz = 0 beside k_press_c, as k_press does it: the integral of H2
+// (linearp.f:172-186, bla/icheb.f) with the constant from E at y = -1, minus E
+static __global__ void __launch_bounds__(128) k_press_mean(PressArgs A, Dims g) {
+  __shared__ double sum[128];
+  const int n = g.nyp, t = threadIdx.x;
+  const size_t NP = g.NP;
+  auto T = [&](int j) { return (j == n - 1 && !A.cim) ? 0.0 : A.CH2[(size_t)j * NP].x; };
+  auto x = [&](int j) {
+    if (j == 1) return T(0) - .5 * T(2);
+    if (j == n - 1) return A.CH2[(size_t)(n - 2) * NP].x * (.5 / (double)(n - 1));
+    return (T(j - 1) - T(j + 1)) * (.5 / (double)j);
+  };
+  double s = 0.0;  // sum over odd j of x_j - x_{j+1}
+  for (int j = t + 1; j < n; j += blockDim.x) {
+    const double v = x(j);
+    s += (j & 1) ? v : -v;
+    const double2 ce = A.CE[(size_t)j * NP];
+    A.X[(size_t)j * NP] = double2{v - ce.x, -ce.y};
+  }
+  sum[t] = s;
+  __syncthreads();
+  if (t == 0) {
+    double x0 = A.PE[(size_t)(n - 1) * NP].x / A.e2n;
+    for (int i = 0; i < (int)blockDim.x; ++i) x0 += sum[i];
+    const double2 ce = A.CE[0];
+    A.X[0] = double2{x0 - ce.x, -ce.y};
+  }
+}
+
+static __global__ void __launch_bounds__(128) k_press(PressArgs A, Dims g) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= g.NP) return;
   const int iz = p / g.nx2;

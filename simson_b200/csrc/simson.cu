@@ -376,10 +376,30 @@ extern "C" const char* sgpu_error_string(int code) {
 
 static size_t smem_fft(int n, int cols, size_t elem) { return 2 * (size_t)n * cols * elem; }
 
+// The chunked kernels' tau coefficients: those of (D^2 - k^2), which do not
+// depend on the time step, are computed here; the per-stage ones (stages) are
+// filled on use.
+static int tau_bufs(sgpu_ctx* c, bool stages) {
+  const Dims& g = c->g;
+  const size_t col = (size_t)g.nyp * (g.nz / 2 + 1) * g.nx2;
+  if (stages && !c->tau_l && cudaMalloc(&c->tau_l, (size_t)c->prm.nst * col * sizeof(double)) != cudaSuccess) {
+    c->tau_l = nullptr;
+    return SGPU_E_CUDA;
+  }
+  if (c->tau_rows) return SGPU_OK;
+  const std::vector<double2> rows = pencil_chunk_table(g.nyp);
+  if ((!c->tau_v && cudaMalloc(&c->tau_v, col * sizeof(double)) != cudaSuccess) ||
+      cudaMalloc(&c->tau_rows, rows.size() * sizeof(double2)) != cudaSuccess)
+    return SGPU_E_CUDA;
+  CK(cudaMemcpyAsync(c->tau_rows, rows.data(), rows.size() * sizeof(double2), cudaMemcpyHostToDevice, c->stream));
+  pencil_tau_coef(c->stream, c->tau_v, g, c->alfa, c->beta, 0.0);
+  CK(cudaStreamSynchronize(c->stream));
+  return SGPU_OK;
+}
+
 // The buffers of the selected pencil kernel (both keep theirs once made): the
 // homogeneous solutions and coefficient columns of the thread-per-pencil
-// kernel, or the tau coefficients of the chunked one, whose (D^2 - k^2) part
-// does not depend on the time step and is computed here.
+// kernel, or the tau coefficients of the chunked one.
 static int pencil_bufs(sgpu_ctx* c) {
   const Dims& g = c->g;
   const size_t fld = (size_t)g.nyp * g.NP, nst = (size_t)c->prm.nst;
@@ -390,17 +410,7 @@ static int pencil_bufs(sgpu_ctx* c) {
       return SGPU_E_CUDA;
     return SGPU_OK;
   }
-  if (!pencil_chunked(c) || c->tau_rows) return SGPU_OK;
-  const size_t col = (size_t)g.nyp * (g.nz / 2 + 1) * g.nx2;
-  const std::vector<double2> rows = pencil_chunk_table(g.nyp);
-  if ((!c->tau_l && cudaMalloc(&c->tau_l, nst * col * sizeof(double)) != cudaSuccess) ||
-      (!c->tau_v && cudaMalloc(&c->tau_v, col * sizeof(double)) != cudaSuccess) ||
-      cudaMalloc(&c->tau_rows, rows.size() * sizeof(double2)) != cudaSuccess)
-    return SGPU_E_CUDA;
-  CK(cudaMemcpyAsync(c->tau_rows, rows.data(), rows.size() * sizeof(double2), cudaMemcpyHostToDevice, c->stream));
-  pencil_tau_coef(c->stream, c->tau_v, g, c->alfa, c->beta, 0.0);
-  CK(cudaStreamSynchronize(c->stream));
-  return SGPU_OK;
+  return pencil_chunked(c) ? tau_bufs(c, true) : SGPU_OK;
 }
 
 extern "C" int sgpu_init(const sgpu_params* prm, sgpu_ctx** out) {
@@ -1807,6 +1817,9 @@ extern "C" int sgpu_pressure(sgpu_ctx* c, double* pr, double* pi) {
   const int n = g.nyp;
   if (n < 9) return SGPU_E_PARAM;
   const size_t fld = (size_t)n * g.NP;
+  // without room for its coefficients the thread-per-pencil kernel solves
+  const bool chunk = pencil_chunk_fits(n) && tau_bufs(c, false) == SGPU_OK;
+  if (!chunk) cudaGetLastError();
   if (!c->press) {
     // second-derivative weights at y = +1 and y = -1 on the Gauss-Lobatto
     // points (bla/preprbl.f:90-118: wd1(:,2) and wd1(:,4))
@@ -1870,7 +1883,12 @@ extern "C" int sgpu_pressure(sgpu_ctx* c, double* pr, double* pi) {
   A.cn = cn;
   A.e2n = 2. * (double)g.nxp * (double)g.nzp;
   A.cim = 0;
-  k_press<<<(g.NP + 127) / 128, 128, 0, c->stream>>>(A, g);
+  if (chunk && press_chunk(c->stream, A, g, c->tau_v, c->tau_rows)) {
+    k_press_mean<<<1, 128, 0, c->stream>>>(A, g);
+    c->launches++;
+  } else {
+    k_press<<<(g.NP + 127) / 128, 128, 0, c->stream>>>(A, g);
+  }
   // back to physical y (vchbb), the oddball plane left out (linearp.f:64)
   launch_cheb_t<double, sgpu_ctx::pb, double, double>(c, czf(c, 7), fld, c->press, fld, 1, 1, 1.0, 1, c->twy.d);
   c->launches += 9;
