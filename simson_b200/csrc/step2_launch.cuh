@@ -14,11 +14,15 @@ namespace sb {
 // threads per CTA of the runtime-plan FFT kernels
 constexpr int SB_FFT_THREADS = 256;
 
-// FP32 transform lengths with compile-time FFT plans (fft.cuh cfft): the
-// production grid's 576 (3/2 x 384) and the test, LES and channel grids' 3/2
-// lengths; any other length takes the runtime plan, and so do all FP64 ones
-// (those of step2_f64.cuh never come here).
-#define SB_FIXED_LENGTHS(X) X(72) X(96) X(240) X(288) X(576)
+// FP32 transform lengths with compile-time FFT plans (fft.cuh cfft): 3/2 of
+// the even products of 2, 3 and 5 that grids are made of, up to 384; any other
+// length takes the runtime plan, and so do all FP64 ones (those of
+// step2_f64.cuh never come here).  Same radices, twiddles and butterflies, so
+// the same results to the last bit.
+#define SB_FIXED_LENGTHS(X)                                                                                          \
+  X(24) X(36) X(48) X(54) X(60) X(72) X(75) X(81) X(90) X(96) X(108) X(120) X(135) X(144) X(150) X(162) X(180)       \
+  X(192) X(216) X(225) X(240) X(270) X(288) X(300) X(324) X(360) X(375) X(384) X(405) X(432) X(450) X(480) X(486)    \
+  X(540) X(576)
 
 // threads per CTA for B columns of an N-point compile-time transform: one
 // butterfly per thread in the widest pass (halved while above 512), a
