@@ -532,9 +532,10 @@ SB_HD __forceinline__ typename C2<T>::type* cfft(typename C2<T>::type* src, type
 // shared memory only between passes.
 // ZM: inputs of the blocks in the mask are zero and not loaded
 // (pad_zero_mask, first pass); DM: outputs of the blocks in the mask are not
-// stored (pad_drop_mask, last pass).
-template <class T, int B, int N, int R, int NS, int S, int NT, unsigned ZM = 0, unsigned DM = 0, class Ld,
-          class St>
+// stored (pad_drop_mask, last pass).  NF: consecutive work items take
+// consecutive elements of one column instead of the columns of one element.
+template <class T, int B, int N, int R, int NS, int S, int NT, unsigned ZM = 0, unsigned DM = 0, bool NF = false,
+          class Ld, class St>
 SB_HD __forceinline__ void cpass_io(Ld ld, St st, const typename C2<T>::type* __restrict__ tw, int t0) {
   typedef typename C2<T>::type V;
   constexpr int nb = N / R;
@@ -545,8 +546,8 @@ SB_HD __forceinline__ void cpass_io(Ld ld, St st, const typename C2<T>::type* __
   for (int it = 0; it < iters; ++it) {
     const int t = t0 + it * NT;
     if (items % NT != 0 && t >= items) break;
-    const unsigned j = (unsigned)t / B;
-    const unsigned b = (unsigned)t - j * B;
+    const unsigned j = NF ? (unsigned)t % nb : (unsigned)t / B;
+    const unsigned b = NF ? (unsigned)t / nb : (unsigned)t - j * B;
     const unsigned jg = j / NS;
     const unsigned jm = j - jg * NS;
     V v[9];
@@ -603,12 +604,14 @@ SB_HD __forceinline__ void cfft_io(Ld ld, St st, typename C2<T>::type* buf0, typ
 }
 
 // First pass from ld, the others in shared memory; returns the buffer that
-// holds the result (ends with a barrier on the device).
-template <class T, int B, int N, int S, int NT, bool ZIN = false, class Ld>
+// holds the result (ends with a barrier on the device).  NF: the first pass's
+// item order (cpass_io), for columns that are contiguous in memory.
+template <class T, int B, int N, int S, int NT, bool ZIN = false, bool NF = false, class Ld>
 SB_HD __forceinline__ typename C2<T>::type* cfft_ld(Ld ld, typename C2<T>::type* buf0, typename C2<T>::type* buf1,
                                                     const typename C2<T>::type* __restrict__ tw, int t0) {
   constexpr CPlanData pl = cplan_make(N);
-  cpass_io<T, B, N, pl.radix[0], pl.ns[0], S, NT, ZIN ? pad_zero_mask<N>() : 0u>(ld, SmemSt<T, B>{buf0}, tw, t0);
+  cpass_io<T, B, N, pl.radix[0], pl.ns[0], S, NT, ZIN ? pad_zero_mask<N>() : 0u, 0u, NF>(ld, SmemSt<T, B>{buf0},
+                                                                                         tw, t0);
 #ifdef __CUDA_ARCH__
   __syncthreads();
 #endif
