@@ -260,7 +260,8 @@ SB_HD __forceinline__ unsigned umulhi_(unsigned a, unsigned b) {
 #ifndef SB_TW_PRODUCTS64
 #define SB_TW_PRODUCTS64 1
 #endif
-template <class T, int R, int S>
+// Q columns of nine values at v share them.
+template <class T, int R, int S, int Q = 1>
 SB_HD __forceinline__ void twiddle(typename C2<T>::type* v, const typename C2<T>::type* __restrict__ tw, int e) {
   typedef typename C2<T>::type V;
   if constexpr (std::is_same<T, float>::value || SB_TW_PRODUCTS64) {
@@ -286,8 +287,11 @@ SB_HD __forceinline__ void twiddle(typename C2<T>::type* v, const typename C2<T>
       w[8] = cmul(w[4], w[4]);
     }
 #pragma unroll
-    for (int r = 1; r < R; ++r) v[r] = cmul(v[r], w[r]);
+    for (int q = 0; q < Q; ++q)
+#pragma unroll
+      for (int r = 1; r < R; ++r) v[9 * q + r] = cmul(v[9 * q + r], w[r]);
   } else {
+    static_assert(Q == 1);
 #pragma unroll
     for (int r = 1; r < R; ++r) {
       V w = tw[r * e];
@@ -472,6 +476,40 @@ constexpr int cplan_max_nb(int n) {
   return mx;
 }
 
+// Columns per work item of the passes in shared memory (cfft, cfft_ld): two
+// neighbouring FP32 columns where B is even, so that a thread computes the
+// indices and the twiddle powers once for both and its accesses are 16 bytes;
+// the values are the same.  Measured in the x pass: n = 288 (192x129x160) 0.193
+// -> 0.160 ms, the step 3.58 -> 3.40.  Not for short lengths, whose CTAs have
+// too few threads then (n = 96: 34 -> 35 us; n = 150: 48 -> 41, but steps of
+// several contexts at once 2.69 -> 2.80 ms), and not for the longest, where
+// four CTAs fill the shared memory and leave other contexts' kernels no place
+// beside them (n = 576: alone 1.01 -> 0.89 ms, three contexts' steps 21.3 -> 21.9).
+// Not in cfft_io either: two columns from and to global memory made the z
+// inverse's accesses 16-byte pieces of a row, 0.51 -> 0.84 ms.
+template <class T, int B, int N>
+constexpr int fft_cols() {
+  return sizeof(T) == 4 && B % 2 == 0 && N >= 240 && N <= 432 ? 2 : 1;
+}
+
+template <class V, int Q>
+SB_HD __forceinline__ void cols_ld(const V* __restrict__ p, V* v) {
+  if constexpr (Q == 2) {
+    const float4 q = *reinterpret_cast<const float4*>(p);
+    v[0] = V{q.x, q.y};
+    v[9] = V{q.z, q.w};
+  } else {
+    v[0] = *p;
+  }
+}
+template <class V, int Q>
+SB_HD __forceinline__ void cols_st(V* __restrict__ p, const V* v) {
+  if constexpr (Q == 2)
+    *reinterpret_cast<float4*>(p) = float4{v[0].x, v[0].y, v[9].x, v[9].y};
+  else
+    *p = v[0];
+}
+
 // One radix-R pass of an N-point transform over B interleaved columns; work
 // items t0, t0 + NT, ...
 // DM: outputs of the blocks in the mask are not stored (pad_drop_mask).
@@ -479,27 +517,29 @@ template <class T, int B, int N, int R, int NS, int S, int NT, unsigned DM = 0>
 SB_HD __forceinline__ void cpass(const typename C2<T>::type* __restrict__ src, typename C2<T>::type* __restrict__ dst,
                                  const typename C2<T>::type* __restrict__ tw, int t0) {
   typedef typename C2<T>::type V;
+  constexpr int Q = fft_cols<T, B, N>();
   constexpr int nb = N / R;
-  constexpr int items = nb * B;
+  constexpr int items = nb * B / Q;
   constexpr int tstep = N / (NS * R);
   constexpr int iters = (items + NT - 1) / NT;
 #pragma unroll
   for (int it = 0; it < iters; ++it) {
     const int t = t0 + it * NT;
     if (items % NT != 0 && t >= items) break;
-    const unsigned j = (unsigned)t / B;
-    const unsigned b = (unsigned)t - j * B;
+    const unsigned j = (unsigned)t / (B / Q);
+    const unsigned b = ((unsigned)t - j * (B / Q)) * Q;
     const unsigned jg = j / NS;
     const unsigned jm = j - jg * NS;
-    V v[9];
+    V v[9 * Q];
 #pragma unroll
-    for (int r = 0; r < R; ++r) v[r] = src[t + r * nb * B];
-    if (NS > 1 && jm != 0) twiddle<T, R, S>(v, tw, (int)(jm * tstep));
-    dft_small<T, V>(v, R, S);
+    for (int r = 0; r < R; ++r) cols_ld<V, Q>(src + t * Q + r * nb * B, v + r);
+    if (NS > 1 && jm != 0) twiddle<T, R, S, Q>(v, tw, (int)(jm * tstep));
+#pragma unroll
+    for (int q = 0; q < Q; ++q) dft_small<T, V>(v + 9 * q, R, S);
     V* __restrict__ d = dst + (size_t)((jg * NS * R + jm) * B + b);
 #pragma unroll
     for (int r = 0; r < R; ++r)
-      if (!(DM & (1u << r))) d[r * NS * B] = v[r];
+      if (!(DM & (1u << r))) cols_st<V, Q>(d + r * NS * B, v + r);
   }
 }
 
@@ -525,43 +565,6 @@ SB_HD __forceinline__ typename C2<T>::type* cfft(typename C2<T>::type* src, type
   }
 }
 
-// One pass with accessors instead of shared-memory buffers: ld(m, b) returns
-// element m of column b of the pass input, st(k, b, v) stores element k of
-// column b of its output.  The first pass of cfft_io reads the global arrays
-// through ld and its last pass writes them through st, so the data crosses
-// shared memory only between passes.
-// ZM: inputs of the blocks in the mask are zero and not loaded
-// (pad_zero_mask, first pass); DM: outputs of the blocks in the mask are not
-// stored (pad_drop_mask, last pass).  NF: consecutive work items take
-// consecutive elements of one column instead of the columns of one element.
-template <class T, int B, int N, int R, int NS, int S, int NT, unsigned ZM = 0, unsigned DM = 0, bool NF = false,
-          class Ld, class St>
-SB_HD __forceinline__ void cpass_io(Ld ld, St st, const typename C2<T>::type* __restrict__ tw, int t0) {
-  typedef typename C2<T>::type V;
-  constexpr int nb = N / R;
-  constexpr int items = nb * B;
-  constexpr int tstep = N / (NS * R);
-  constexpr int iters = (items + NT - 1) / NT;
-#pragma unroll
-  for (int it = 0; it < iters; ++it) {
-    const int t = t0 + it * NT;
-    if (items % NT != 0 && t >= items) break;
-    const unsigned j = NF ? (unsigned)t % nb : (unsigned)t / B;
-    const unsigned b = NF ? (unsigned)t / nb : (unsigned)t - j * B;
-    const unsigned jg = j / NS;
-    const unsigned jm = j - jg * NS;
-    V v[9];
-#pragma unroll
-    for (int r = 0; r < R; ++r) v[r] = (ZM & (1u << r)) ? V{(T)0, (T)0} : ld((int)(j + r * nb), (int)b);
-    if (NS > 1 && jm != 0) twiddle<T, R, S>(v, tw, (int)(jm * tstep));
-    dft_small_z<T, V, ZM>(v, R, S);
-    const int k0 = (int)(jg * NS * R + jm);
-#pragma unroll
-    for (int r = 0; r < R; ++r)
-      if (!(DM & (1u << r))) st(k0 + r * NS, (int)b, v[r]);
-  }
-}
-
 template <class T, int B>
 struct SmemLd {
   const typename C2<T>::type* __restrict__ p;
@@ -572,6 +575,57 @@ struct SmemSt {
   typename C2<T>::type* __restrict__ p;
   SB_HD __forceinline__ void operator()(int k, int b, typename C2<T>::type v) const { p[k * B + b] = v; }
 };
+
+// One pass with accessors instead of shared-memory buffers: ld(m, b) returns
+// element m of column b of the pass input, st(k, b, v) stores element k of
+// column b of its output.  The first pass of cfft_io reads the global arrays
+// through ld and its last pass writes them through st, so the data crosses
+// shared memory only between passes.
+// ZM: inputs of the blocks in the mask are zero and not loaded
+// (pad_zero_mask, first pass); DM: outputs of the blocks in the mask are not
+// stored (pad_drop_mask, last pass).  NF: consecutive work items take
+// consecutive elements of one column instead of the columns of one element.
+// Q: columns per item.
+template <class T, int B, int N, int R, int NS, int S, int NT, unsigned ZM = 0, unsigned DM = 0, bool NF = false,
+          int Q = 1, class Ld, class St>
+SB_HD __forceinline__ void cpass_io(Ld ld, St st, const typename C2<T>::type* __restrict__ tw, int t0) {
+  typedef typename C2<T>::type V;
+  constexpr int nb = N / R;
+  constexpr int items = nb * B / Q;
+  constexpr int tstep = N / (NS * R);
+  constexpr int iters = (items + NT - 1) / NT;
+#pragma unroll
+  for (int it = 0; it < iters; ++it) {
+    const int t = t0 + it * NT;
+    if (items % NT != 0 && t >= items) break;
+    const unsigned j = NF ? (unsigned)t % nb : (unsigned)t / (B / Q);
+    const unsigned b = (NF ? (unsigned)t / nb : (unsigned)t - j * (B / Q)) * Q;
+    const unsigned jg = j / NS;
+    const unsigned jm = j - jg * NS;
+    V v[9 * Q];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      if constexpr (Q == 2 && std::is_same<Ld, SmemLd<T, B>>::value)
+        cols_ld<V, Q>(ld.p + ((int)j + r * nb) * B + (int)b, v + r);
+      else
+#pragma unroll
+        for (int q = 0; q < Q; ++q) v[9 * q + r] = (ZM & (1u << r)) ? V{(T)0, (T)0} : ld((int)(j + r * nb), (int)b + q);
+    }
+    if (NS > 1 && jm != 0) twiddle<T, R, S, Q>(v, tw, (int)(jm * tstep));
+#pragma unroll
+    for (int q = 0; q < Q; ++q) dft_small_z<T, V, ZM>(v + 9 * q, R, S);
+    const int k0 = (int)(jg * NS * R + jm);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      if (DM & (1u << r)) continue;
+      if constexpr (Q == 2 && std::is_same<St, SmemSt<T, B>>::value)
+        cols_st<V, Q>(st.p + (k0 + r * NS) * B + (int)b, v + r);
+      else
+#pragma unroll
+        for (int q = 0; q < Q; ++q) st(k0 + r * NS, (int)b + q, v[9 * q + r]);
+    }
+  }
+}
 
 // N-point transform of B columns from ld to st (at least two passes);
 // buf0/buf1 hold the intermediate passes.  The caller syncs before reusing
@@ -610,7 +664,7 @@ template <class T, int B, int N, int S, int NT, bool ZIN = false, bool NF = fals
 SB_HD __forceinline__ typename C2<T>::type* cfft_ld(Ld ld, typename C2<T>::type* buf0, typename C2<T>::type* buf1,
                                                     const typename C2<T>::type* __restrict__ tw, int t0) {
   constexpr CPlanData pl = cplan_make(N);
-  cpass_io<T, B, N, pl.radix[0], pl.ns[0], S, NT, ZIN ? pad_zero_mask<N>() : 0u, 0u, NF>(ld, SmemSt<T, B>{buf0},
+  cpass_io<T, B, N, pl.radix[0], pl.ns[0], S, NT, ZIN ? pad_zero_mask<N>() : 0u, 0u, NF, fft_cols<T, B, N>()>(ld, SmemSt<T, B>{buf0},
                                                                                          tw, t0);
 #ifdef __CUDA_ARCH__
   __syncthreads();

@@ -24,11 +24,11 @@ constexpr int SB_FFT_THREADS = 256;
   X(192) X(216) X(225) X(240) X(270) X(288) X(300) X(324) X(360) X(375) X(384) X(405) X(432) X(450) X(480) X(486)    \
   X(540) X(576)
 
-// threads per CTA for B columns of an N-point compile-time transform: one
-// butterfly per thread in the widest pass (halved while above 512), a
-// multiple of 32
-constexpr int fixed_threads(int n, int b) {
-  int items = cplan_max_nb(n) * b;
+// threads per CTA for B columns, Q per work item, of an N-point compile-time
+// transform: one item per thread in the widest pass (halved while above 512),
+// a multiple of 32
+constexpr int fixed_threads(int n, int b, int q = 1) {
+  int items = cplan_max_nb(n) * b / q;
   while (items > 512) items = (items + 1) / 2;
   return ((items + 31) / 32) * 32;
 }
@@ -101,8 +101,8 @@ inline void launch_xpass(dim3 grid, size_t smem, cudaStream_t st, const typename
 #define SB_CASE(n)                                                                                                \
   case n:                                                                                                         \
     if constexpr (sizeof(T) == 4)                                                                                 \
-      xpass_n<T, RB, n, fixed_threads(n, 3 * RB)>(grid, smem, st, zb, xb, g, plan, tw, dyi, dxi, dzi, rot, cfl,    \
-                                                  mean, fr);                                                      \
+      xpass_n<T, RB, n, fixed_threads(n, 3 * RB, fft_cols<T, 3 * RB, n>())>(grid, smem, st, zb, xb, g, plan, tw,   \
+                                                                            dyi, dxi, dzi, rot, cfl, mean, fr);    \
     return;
     SB_FIXED_LENGTHS(SB_CASE)
 #undef SB_CASE
