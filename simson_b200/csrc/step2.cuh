@@ -40,8 +40,8 @@ __device__ __forceinline__ void z_prefetch_l2(const void* ptr) {
 // Omega_x, Omega_z), which the mixed-precision path adds back analytically.
 // N > 0: the z length g.nzp is N, transformed with the compile-time plan by
 // NT threads per CTA; N = 0: runtime plan, any block size.
-// (the FP64 fixed-length variant is held to three CTAs per SM: unbounded it
-// takes ~130 registers and one CTA per SM)
+// (FP64, the lengths without a two-pass kernel (step2_f64.cuh), is held to three
+// CTAs per SM: unbounded it takes ~130 registers and one CTA per SM)
 // SB_ZINV_MINB, SB_ZFWD_MINB: the same for the FP32 variants of the long
 // transforms (N >= 288).  Four CTAs per SM (z-inverse 62 -> 55 registers,
 // z-forward 94 -> 52, no spills) measured faster than the compiler's choice
@@ -53,8 +53,6 @@ __device__ __forceinline__ void z_prefetch_l2(const void* ptr) {
 #ifndef SB_ZFWD_MINB
 #define SB_ZFWD_MINB 4
 #endif
-// SB_ZINV64_MINB: the FP64 variant (three CTAs of 288 threads at 72
-// registers; four, at 56, measured 1.116 -> 1.148 ms at 384x193x384)
 #ifndef SB_ZINV64_MINB
 #define SB_ZINV64_MINB 3
 #endif
@@ -167,15 +165,9 @@ __device__ __forceinline__ void fringe_apply(const Fringe& fr, int j, int y, int
 #ifndef SB_XPASS_MINB
 #define SB_XPASS_MINB 0
 #endif
-// SB_XPASS64_MINB: the same for the FP64 fixed-length variant (0: the
-// compiler's choice, four CTAs of 224 threads at 66 registers; five, at 56
-// registers and a 20-byte spill, measured 2.24 -> 2.34 ms at 384x193x384)
-#ifndef SB_XPASS64_MINB
-#define SB_XPASS64_MINB 0
-#endif
 template <class T, int RB, int N = 0, int NT = 0>
 __global__ void __launch_bounds__(NT > 0 ? NT : 256,
-                                  NT > 0 ? (sizeof(T) == 4 ? SB_XPASS_MINB : SB_XPASS64_MINB) : 0)
+                                  NT > 0 && sizeof(T) == 4 ? SB_XPASS_MINB : 0)
     k_xpass(const typename C2<T>::type* __restrict__ zb, typename C2<T>::type* __restrict__ xb, Dims g,
             FFTPlan plan, const typename C2<T>::type* __restrict__ tw, const double* __restrict__ dyi, double dxi,
             double dzi, double rot, unsigned long long* __restrict__ cfl_bits, const double* __restrict__ mean,
@@ -319,8 +311,7 @@ __global__ void __launch_bounds__(NT > 0 ? NT : 256,
 
 // mean != nullptr: add nxp*nzp*(W Omega_x - U (Omega_z + 2 rot)) to the
 // kx = kz = 0 mode of H2 in FP64 (the mean-mean product left out by k_xpass).
-// FP64 z-forward: three CTAs per SM (102 -> 72 registers, an 8-byte spill)
-// measured 0.710 -> 0.633 ms at 384x193x384 against the compiler's two
+// FP64, as in k_zinv: three CTAs per SM
 #ifndef SB_ZFWD64_MINB
 #define SB_ZFWD64_MINB 3
 #endif
