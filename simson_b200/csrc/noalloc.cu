@@ -39,6 +39,7 @@
 #include "../../include/simson_b200.h"
 #include "fft.cuh"
 #include "layout.cuh"
+#include "smem.h"
 #include "step2.cuh"
 
 using namespace sb;
@@ -166,12 +167,8 @@ extern "C" int sgpu_nonlin_noalloc(const sgpu_params* prm, const void* fields_in
   const size_t s_z = 2 * (size_t)g.nzp * KB * sizeof(double2);
   const size_t s_x = 2 * (size_t)g.nxp * 3 * RB * sizeof(double2);
   if (s_z > 227 * 1024 || s_x > 227 * 1024) return SGPU_E_PARAM;
-  if (cudaFuncSetAttribute(k_zinv<double, KB, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s_z) !=
-          cudaSuccess ||
-      cudaFuncSetAttribute(k_zfwd<double, KB, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s_z) !=
-          cudaSuccess ||
-      cudaFuncSetAttribute(k_xpass<double, RB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s_x) !=
-          cudaSuccess) {
+  if (smem_max(k_zinv<double, KB, double>) != cudaSuccess || smem_max(k_zfwd<double, KB, double>) != cudaSuccess ||
+      smem_max(k_xpass<double, RB>) != cudaSuccess) {
     fprintf(stderr, "simson_b200: sgpu_nonlin_noalloc: shared-memory opt-in refused: %s\n",
             cudaGetErrorString(cudaGetLastError()));
     return SGPU_E_CUDA;

@@ -33,6 +33,7 @@
 #include "cheb_tc.cuh"
 #include "pencil_chunk.h"
 #include "pencil_warp.cuh"
+#include "smem.h"
 
 using namespace sb;
 
@@ -516,15 +517,11 @@ extern "C" int sgpu_init(const sgpu_params* prm, sgpu_ctx** out) {
   if (s_z > 227 * 1024 || s_x > 227 * 1024 || s_y > 227 * 1024 || s_zf > 227 * 1024 || s_xf > 227 * 1024 ||
       s_yf > 227 * 1024)
     return fail(SGPU_E_PARAM);
-  cudaFuncSetAttribute(k_cheb<double, sgpu_ctx::pb, double, double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)s_y);
+  smem_max(k_cheb<double, sgpu_ctx::pb, double, double>);
   // FP32 variants (their own tiles)
-  cudaFuncSetAttribute(k_cheb<float, sgpu_ctx::pbf, float, double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)s_yf);
-  cudaFuncSetAttribute(k_cheb<float, sgpu_ctx::pbf, double, float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)s_yf);
-  cudaFuncSetAttribute(k_cheb<float, sgpu_ctx::pbf, float, float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)s_yf);
+  smem_max(k_cheb<float, sgpu_ctx::pbf, float, double>);
+  smem_max(k_cheb<float, sgpu_ctx::pbf, double, float>);
+  smem_max(k_cheb<float, sgpu_ctx::pbf, float, float>);
   c->dtn = P.dt;
   c->dt_next = P.dt;
   // SIMSON_GRAPHS=0: launch every kernel directly (no CUDA-graph replay)
@@ -1685,13 +1682,13 @@ static int xys_setup(sgpu_ctx* c) {
     return SGPU_E_CUDA;
   CK(cudaMemsetAsync(c->xys, 0, XYS_NS * plane * sizeof(double), c->stream));
   c->xys_sumw = 0.0;
-  cudaFuncSetAttribute(k_xys_zinv<double2, KB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sz);
-  cudaFuncSetAttribute(k_xys_zinv<float2, KB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sz);
-  cudaFuncSetAttribute(k_xys_acc<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sx);
-  cudaFuncSetAttribute(k_xys_acc<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sx);
-  cudaFuncSetAttribute(k_xys_acc<false, 384>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sx);
-  cudaFuncSetAttribute(k_xys_acc<true, 384>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sx);
-  cudaFuncSetAttribute(k_box_sample, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sx);
+  smem_max(k_xys_zinv<double2, KB>);
+  smem_max(k_xys_zinv<float2, KB>);
+  smem_max(k_xys_acc<false>);
+  smem_max(k_xys_acc<true>);
+  smem_max(k_xys_acc<false, 384>);
+  smem_max(k_xys_acc<true, 384>);
+  smem_max(k_box_sample);
   return SGPU_OK;
 }
 
@@ -1860,7 +1857,7 @@ extern "C" int sgpu_pressure(sgpu_ctx* c, double* pr, double* pi) {
   zinv64(c, g, c->mixed);
   if (!f2_xpass_p(c->stream, c->zb, g, c->twx.d, P.rot, ctx_fringe(c))) {
     const size_t s_xp = 2 * (size_t)g.nxp * 3 * sizeof(double2);
-    cudaFuncSetAttribute(k_xpass_p, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s_xp);
+    smem_max(k_xpass_p);
     k_xpass_p<<<dim3(g.nzp, n), 256, s_xp, c->stream>>>(c->zb, g, c->twx.plan, c->twx.d, P.rot, ctx_fringe(c));
   }
   const size_t fz = (size_t)n * g.nzp * g.nx2;  // one field of zb
@@ -2066,16 +2063,14 @@ static int sgs_setup(sgpu_ctx* c) {
       return SGPU_E_CUDA;
     int rg = les_gu_ensure(c, 3);
     if (rg) return rg;
-    const int sm[4] = {(int)sz, (int)sx11, (int)(2 * (size_t)g.nx * 3 * sizeof(double2)),
-                       (int)(2 * (size_t)g.nx * 5 * sizeof(double2))};
-    cudaFuncSetAttribute(k_sgs_zinv<double2, KB>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm[0]);
-    cudaFuncSetAttribute(k_sgs_zinv<float2, KB>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm[0]);
-    cudaFuncSetAttribute(k_sgs_zfilt<KB>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm[0]);
-    cudaFuncSetAttribute(k_sgs_zfwd<KB>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm[0]);
-    cudaFuncSetAttribute(k_sgs_xpass1, cudaFuncAttributeMaxDynamicSharedMemorySize, sm[1]);
-    cudaFuncSetAttribute(k_sgs_xpass2, cudaFuncAttributeMaxDynamicSharedMemorySize, sm[1]);
-    cudaFuncSetAttribute(k_sgs_tau_x, cudaFuncAttributeMaxDynamicSharedMemorySize, sm[2]);
-    cudaFuncSetAttribute(k_sgs_xinv9, cudaFuncAttributeMaxDynamicSharedMemorySize, sm[3]);
+    smem_max(k_sgs_zinv<double2, KB>);
+    smem_max(k_sgs_zinv<float2, KB>);
+    smem_max(k_sgs_zfilt<KB>);
+    smem_max(k_sgs_zfwd<KB>);
+    smem_max(k_sgs_xpass1);
+    smem_max(k_sgs_xpass2);
+    smem_max(k_sgs_tau_x);
+    smem_max(k_sgs_xinv9);
   }
   // Delta^2 = (dx dz dy)^(2/3), dy the geometric mean of the two
   // neighbouring Gauss-Lobatto spacings, 1 - eta_2 at the walls
@@ -2298,9 +2293,8 @@ extern "C" int sgpu_set_les(sgpu_ctx* c, const sgpu_les_params* p) {
     }
     CK(cudaMemcpyAsync(c->les_hmat, M.data(), M.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream));
     CK(cudaStreamSynchronize(c->stream));
-    const int sm = les_hpf_smem(g.nyp);
-    cudaFuncSetAttribute(k_les_hpf2<float2>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-    cudaFuncSetAttribute(k_les_hpf2<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+    smem_max(k_les_hpf2<float2>);
+    smem_max(k_les_hpf2<double2>);
   }
   c->les_fact2 = F.fact2;
   c->les_factm2 = F.factm2;

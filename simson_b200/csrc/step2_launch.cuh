@@ -7,6 +7,7 @@
 
 #include "fft.cuh"
 #include "layout.cuh"
+#include "smem.h"
 #include "step2.cuh"
 
 namespace sb {
@@ -33,11 +34,20 @@ constexpr int fixed_threads(int n, int b, int q = 1) {
   return ((items + 31) / 32) * 32;
 }
 
+// the runtime plan's instance serves every other length, the others one each
+template <int N, class K>
+inline void smem_limit(K kernel, size_t smem) {
+  if constexpr (N > 0)
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  else
+    smem_max(kernel);
+}
+
 template <class T, int KB, class S, int N, int NT>
 inline void zinv_n(dim3 grid, size_t smem, cudaStream_t st, const typename C2<S>::type* in,
                    typename C2<T>::type* zb, const Dims& g, const FFTPlan& plan, const typename C2<T>::type* tw,
                    const double* alfa, const double* beta, int drop) {
-  cudaFuncSetAttribute(k_zinv<T, KB, S, N, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  smem_limit<N>(k_zinv<T, KB, S, N, NT>, smem);
   k_zinv<T, KB, S, N, NT><<<grid, NT, smem, st>>>(in, zb, g, plan, tw, alfa, beta, drop);
 }
 template <class T, int KB, class S>
@@ -61,7 +71,7 @@ template <class T, int KB, class S, int N, int NT>
 inline void zfwd_n(dim3 grid, size_t smem, cudaStream_t st, const typename C2<T>::type* xb,
                    typename C2<S>::type* out, const Dims& g, const FFTPlan& plan, const typename C2<T>::type* tw,
                    const double* mean, double rot) {
-  cudaFuncSetAttribute(k_zfwd<T, KB, S, N, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  smem_limit<N>(k_zfwd<T, KB, S, N, NT>, smem);
   k_zfwd<T, KB, S, N, NT><<<grid, NT, smem, st>>>(xb, out, g, plan, tw, mean, rot);
 }
 template <class T, int KB, class S>
@@ -86,7 +96,7 @@ inline void xpass_n(dim3 grid, size_t smem, cudaStream_t st, const typename C2<T
                     typename C2<T>::type* xb, const Dims& g, const FFTPlan& plan, const typename C2<T>::type* tw,
                     const double* dyi, double dxi, double dzi, double rot, unsigned long long* cfl,
                     const double* mean, Fringe fr) {
-  cudaFuncSetAttribute(k_xpass<T, RB, N, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  smem_limit<N>(k_xpass<T, RB, N, NT>, smem);
 #ifdef SB_XPASS_CARVEOUT
   cudaFuncSetAttribute(k_xpass<T, RB, N, NT>, cudaFuncAttributePreferredSharedMemoryCarveout, SB_XPASS_CARVEOUT);
 #endif
