@@ -333,7 +333,8 @@ int sgpu_cfl_set_global(sgpu_ctx* ctx, double cflp);
  * above 8192 pencils (nz nx/2) (the default, also set at sgpu_init;
  * SIMSON_PENCIL_WARP=0/1 in the environment forces one for new contexts).
  * All solve the same tau systems, to round-off.  SGPU_E_PARAM for warp = 1
- * when ny > 256. */
+ * when ny > 256.  A kernel's buffers are made when it is first selected:
+ * SGPU_E_CUDA when there is no room for them, and the former kernel stays. */
 int sgpu_set_pencil_kernel(sgpu_ctx* ctx, int warp);
 
 /* Failure detection of the tensor-core kernels (the mixed path's Chebyshev

@@ -101,6 +101,7 @@ struct sgpu_ctx {
   double* tau_l = nullptr;
   double* tau_v = nullptr;
   double2* tau_rows = nullptr;
+  bool tau_ready = false;  // tau_v and tau_rows are filled
   double tau_key[4] = {0.0, 0.0, 0.0, 0.0};
   int tau_next = 0;
   double* mscr = nullptr;    // mean-flow scratch
@@ -377,40 +378,45 @@ extern "C" const char* sgpu_error_string(int code) {
 
 static size_t smem_fft(int n, int cols, size_t elem) { return 2 * (size_t)n * cols * elem; }
 
+// A device buffer made on first use.  A refused one leaves no error behind for
+// the next launch check to find.
+template <class T>
+static bool ensure(T*& p, size_t count) {
+  if (p) return true;
+  if (cudaMalloc(&p, count * sizeof(T)) == cudaSuccess) return true;
+  p = nullptr;
+  cudaGetLastError();
+  return false;
+}
+
 // The chunked kernels' tau coefficients: those of (D^2 - k^2), which do not
 // depend on the time step, are computed here; the per-stage ones (stages) are
 // filled on use.
 static int tau_bufs(sgpu_ctx* c, bool stages) {
   const Dims& g = c->g;
   const size_t col = (size_t)g.nyp * (g.nz / 2 + 1) * g.nx2;
-  if (stages && !c->tau_l && cudaMalloc(&c->tau_l, (size_t)c->prm.nst * col * sizeof(double)) != cudaSuccess) {
-    c->tau_l = nullptr;
-    return SGPU_E_CUDA;
-  }
-  if (c->tau_rows) return SGPU_OK;
+  if (stages && !ensure(c->tau_l, (size_t)c->prm.nst * col)) return SGPU_E_CUDA;
+  if (c->tau_ready) return SGPU_OK;
   const std::vector<double2> rows = pencil_chunk_table(g.nyp);
-  if ((!c->tau_v && cudaMalloc(&c->tau_v, col * sizeof(double)) != cudaSuccess) ||
-      cudaMalloc(&c->tau_rows, rows.size() * sizeof(double2)) != cudaSuccess)
-    return SGPU_E_CUDA;
+  if (!ensure(c->tau_v, col) || !ensure(c->tau_rows, rows.size())) return SGPU_E_CUDA;
   CK(cudaMemcpyAsync(c->tau_rows, rows.data(), rows.size() * sizeof(double2), cudaMemcpyHostToDevice, c->stream));
   pencil_tau_coef(c->stream, c->tau_v, g, c->alfa, c->beta, 0.0);
+  CK(cudaGetLastError());
   CK(cudaStreamSynchronize(c->stream));
+  c->tau_ready = true;
   return SGPU_OK;
 }
 
-// The buffers of the selected pencil kernel (both keep theirs once made): the
-// homogeneous solutions and coefficient columns of the thread-per-pencil
-// kernel, or the tau coefficients of the chunked one.
-static int pencil_bufs(sgpu_ctx* c) {
+// The buffers of a pencil kernel (both keep theirs once made): the homogeneous
+// solutions and coefficient columns of the thread-per-pencil kernel, or the
+// tau coefficients of the chunked one (group).
+static int pencil_bufs(sgpu_ctx* c, bool group) {
   const Dims& g = c->g;
   const size_t fld = (size_t)g.nyp * g.NP, nst = (size_t)c->prm.nst;
-  if (!c->pencil_group) {
-    if ((!c->hom_vh && cudaMalloc(&c->hom_vh, nst * fld * sizeof(double)) != cudaSuccess) ||
-        (!c->hom_s && cudaMalloc(&c->hom_s, nst * 2 * (size_t)g.NP * sizeof(double)) != cudaSuccess) ||
-        (!c->hom_cf && cudaMalloc(&c->hom_cf, nst * 4 * fld * sizeof(double)) != cudaSuccess))
-      return SGPU_E_CUDA;
-    return SGPU_OK;
-  }
+  if (!group)
+    return ensure(c->hom_vh, nst * fld) && ensure(c->hom_s, nst * 2 * (size_t)g.NP) && ensure(c->hom_cf, nst * 4 * fld)
+               ? SGPU_OK
+               : SGPU_E_CUDA;
   return pencil_chunked(c) ? tau_bufs(c, true) : SGPU_OK;
 }
 
@@ -530,7 +536,7 @@ extern "C" int sgpu_init(const sgpu_params* prm, sgpu_ctx** out) {
   // SIMSON_PENCIL_WARP=0/1 forces one of step 3's pencil kernels
   const char* pw = getenv("SIMSON_PENCIL_WARP");
   c->pencil_group = pw ? (pw[0] == '1' && pencil_group_fits(c)) : pencil_group_auto(c);
-  if ((rc = pencil_bufs(c))) return fail(rc);
+  if ((rc = pencil_bufs(c, c->pencil_group))) return fail(rc);
   if (cudaDeviceSynchronize() != cudaSuccess) return fail(SGPU_E_CUDA);
   *out = c;
   return SGPU_OK;
@@ -1584,8 +1590,11 @@ extern "C" int sgpu_set_pencil_kernel(sgpu_ctx* c, int warp) {
   if (c) c->step_valid = false;  // the captured step launches the other kernel
   if (!c || warp < 0 || warp > 2) return SGPU_E_PARAM;
   if (warp == 1 && c->g.nyp > 256) return SGPU_E_PARAM;
-  c->pencil_group = warp == 2 ? pencil_group_auto(c) : (warp == 1 && pencil_group_fits(c));
-  return pencil_bufs(c);
+  const bool group = warp == 2 ? pencil_group_auto(c) : (warp == 1 && pencil_group_fits(c));
+  // its buffers first: without room for them the former kernel stays selected
+  const int rc = pencil_bufs(c, group);
+  if (rc == SGPU_OK) c->pencil_group = group;
+  return rc;
 }
 
 extern "C" int sgpu_set_wait_limit(sgpu_ctx* c, int limit, int test_timeout) {
@@ -1819,7 +1828,6 @@ extern "C" int sgpu_pressure(sgpu_ctx* c, double* pr, double* pi) {
   const size_t fld = (size_t)n * g.NP;
   // without room for its coefficients the thread-per-pencil kernel solves
   const bool chunk = pencil_chunk_fits(n) && tau_bufs(c, false) == SGPU_OK;
-  if (!chunk) cudaGetLastError();
   if (!c->press) {
     // second-derivative weights at y = +1 and y = -1 on the Gauss-Lobatto
     // points (bla/preprbl.f:90-118: wd1(:,2) and wd1(:,4))
