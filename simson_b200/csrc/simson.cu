@@ -851,7 +851,7 @@ static void les_filter_velocity(sgpu_ctx* c, int skip_oddball) {
   const int nf = c->iles == 3 ? 5 : 3;
   prof_mark(c, K_OTHER);
   auto filter = [&](double2* gu, const double* lpf, const double* filt) {
-    if (c->les_mode == 2 && les_hpf_fits(g.nyp)) {
+    if (c->les_mode == 2 && c->les_hmat) {
       const dim3 grid((g.NP + LES_TP - 1) / LES_TP, nf);
       const int nt = les_hpf_threads(g.nyp), sm = les_hpf_smem(g.nyp);
       if (c->mixed)
@@ -2291,16 +2291,15 @@ extern "C" int sgpu_set_les(sgpu_ctx* c, const sgpu_les_params* p) {
                      c->stream));
   CK(cudaStreamSynchronize(c->stream));
   if (p->ihighorder == 2 && les_hpf_fits(g.nyp)) {
-    // the wall-normal matrix of the tensorial filter
+    // the wall-normal matrix of the tensorial filter; without room for it the
+    // column solves (k_les_hpf) filter
     YFilter Y{rows.data(), F.fact2, F.factm2, g.nyp};
     std::vector<double> M;
     les_hpf_matrix(Y, p->iord, M);
-    if (!c->les_hmat && cudaMalloc(&c->les_hmat, M.size() * sizeof(double)) != cudaSuccess) {
-      c->les_hmat = nullptr;  // (the matrix's size depends on ny only)
-      return SGPU_E_CUDA;
+    if (ensure(c->les_hmat, M.size())) {  // (the matrix's size depends on ny only)
+      CK(cudaMemcpyAsync(c->les_hmat, M.data(), M.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+      CK(cudaStreamSynchronize(c->stream));
     }
-    CK(cudaMemcpyAsync(c->les_hmat, M.data(), M.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
     smem_max(k_les_hpf2<float2>);
     smem_max(k_les_hpf2<double2>);
   }
