@@ -61,27 +61,29 @@ __global__ void __launch_bounds__(f2_threads(F2<N, LF_KB>::items))
 }
 
 // Row f of the statistics from the eight spectra: (r0 + i c0 alpha) q_s0 + r1
-// q_s1, packed as s0 + 16 s1 + 256 (r0 + 1) + 1024 (c0 + 1) + 4096 (r1 + 1)
+// q_s1, packed as s0 + 16 s1 + 256 (r0 + 1) + 1024 (c0 + 1) + 4096 (r1 + 1).  A
+// row of one spectrum names it twice: zero times another one would carry that
+// one's infinities and NaN into it.
 constexpr int xys_row(int s0, int r0, int c0, int s1, int r1) {
   return s0 + 16 * s1 + 256 * (r0 + 1) + 1024 * (c0 + 1) + 4096 * (r1 + 1);
 }
 __device__ __constant__ const int kXysRow[16] = {
     xys_row(0, 1, 0, 0, 0),    // u
-    xys_row(1, 1, 0, 0, 0),    // v
-    xys_row(2, 1, 0, 0, 0),    // w
-    xys_row(3, 1, 0, 0, 0),    // omega_x
+    xys_row(1, 1, 0, 1, 0),    // v
+    xys_row(2, 1, 0, 2, 0),    // w
+    xys_row(3, 1, 0, 3, 0),    // omega_x
     xys_row(2, 0, -1, 5, 1),   // omega_y = du/dz - dw/dx
-    xys_row(4, 1, 0, 0, 0),    // omega_z
+    xys_row(4, 1, 0, 4, 0),    // omega_z
     xys_row(0, 0, 1, 0, 0),    // du/dx
     xys_row(1, 0, 1, 4, -1),   // du/dy = dv/dx - omega_z
-    xys_row(5, 1, 0, 0, 0),    // du/dz
-    xys_row(1, 0, 1, 0, 0),    // dv/dx
+    xys_row(5, 1, 0, 5, 0),    // du/dz
+    xys_row(1, 0, 1, 1, 0),    // dv/dx
     xys_row(0, 0, -1, 7, -1),  // dv/dy = -du/dx - dw/dz
-    xys_row(6, 1, 0, 0, 0),    // dv/dz
-    xys_row(2, 0, 1, 0, 0),    // dw/dx
+    xys_row(6, 1, 0, 6, 0),    // dv/dz
+    xys_row(2, 0, 1, 2, 0),    // dw/dx
     xys_row(3, 1, 0, 6, 1),    // dw/dy = omega_x + dv/dz
-    xys_row(7, 1, 0, 0, 0),    // dw/dz
-    xys_row(8, 1, 0, 0, 0),    // p
+    xys_row(7, 1, 0, 7, 0),    // dw/dz
+    xys_row(8, 1, 0, 8, 0),    // p
 };
 
 constexpr int XYS_XT = 128;  // threads of k_xys_x15
