@@ -6,7 +6,8 @@
 // device memory is managed by its own pool, or a host that has already
 // reserved (nearly) all of the GPU's memory for its fields.  Such a caller
 // passes its own device input and output arrays and gets the same kernels as
-// sgpu_nonlin, with the two intermediate buffers of the step (the z-transformed
+// sgpu_nonlin (the two-pass transforms of step2_f64.cuh where the length has
+// them), with the two intermediate buffers of the step (the z-transformed
 // fields and the x-transformed products) and the small tables (twiddles,
 // wavenumbers, CFL grid spacing) placed in one file-scope static device array.
 //
@@ -41,6 +42,7 @@
 #include "layout.cuh"
 #include "smem.h"
 #include "step2.cuh"
+#include "step2_f64.h"
 
 using namespace sb;
 
@@ -163,6 +165,8 @@ extern "C" int sgpu_nonlin_noalloc(const sgpu_params* prm, const void* fields_in
   // the CFL word starts at zero every call
   if (cudaMemsetAsync(cfl_bits, 0, sizeof(unsigned long long), st) != cudaSuccess) return SGPU_E_CUDA;
 
+  // the passes of sgpu_nonlin: the two-pass kernels where the length has one,
+  // the Stockham kernels with the runtime plan elsewhere
   constexpr int KB = 4, RB = 1, TH = 128;
   const size_t s_z = 2 * (size_t)g.nzp * KB * sizeof(double2);
   const size_t s_x = 2 * (size_t)g.nxp * 3 * RB * sizeof(double2);
@@ -175,14 +179,15 @@ extern "C" int sgpu_nonlin_noalloc(const sgpu_params* prm, const void* fields_in
   }
   const double2* in = static_cast<const double2*>(fields_in);
   double2* out = static_cast<double2*>(h_out);
-  dim3 gz((g.nx2 + KB - 1) / KB, g.nyp);
-  k_zinv<double, KB, double><<<gz, TH, s_z, st>>>(in, zb, g, pz, twz, alfa, beta, 0);
-  dim3 gx((g.nzp + RB - 1) / RB, g.nyp);
+  const dim3 gz((g.nx2 + KB - 1) / KB, g.nyp), gx((g.nzp + RB - 1) / RB, g.nyp);
   const double dxi = (double)(g.nx - 2) / P.xl;
   const double dzi = (double)(g.nz - 2) / P.zl;
-  k_xpass<double, RB><<<gx, TH, s_x, st>>>(zb, xb, g, px, twx, dyi, dxi, dzi, P.rot, cfl_bits, nullptr,
-                                          Fringe{nullptr, nullptr});
-  k_zfwd<double, KB, double><<<gz, TH, s_z, st>>>(xb, out, g, pz, twz, nullptr, 0.0);
+  const Fringe none{nullptr, nullptr};
+  if (!f2_zinv(st, in, nullptr, zb, g, twz, alfa, beta))
+    k_zinv<double, KB, double><<<gz, TH, s_z, st>>>(in, zb, g, pz, twz, alfa, beta, 0);
+  if (!f2_xpass(st, zb, xb, g, twx, dyi, dxi, dzi, P.rot, cfl_bits, none))
+    k_xpass<double, RB><<<gx, TH, s_x, st>>>(zb, xb, g, px, twx, dyi, dxi, dzi, P.rot, cfl_bits, nullptr, none);
+  if (!f2_zfwd(st, xb, out, g, twz)) k_zfwd<double, KB, double><<<gz, TH, s_z, st>>>(xb, out, g, pz, twz, nullptr, 0.0);
   if (cudaGetLastError() != cudaSuccess) return SGPU_E_CUDA;
   if (cflp_max) {
     unsigned long long bits = 0;

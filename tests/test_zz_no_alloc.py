@@ -55,3 +55,40 @@ def test_nonlin_noalloc_matches_sgpu_nonlin():
     assert lib.sgpu_nonlin_noalloc(ctypes.byref(big), ctypes.c_void_p(dev_in.data_ptr()),
                                    ctypes.c_void_p(out.data_ptr()), None, None) == -1
     ch.close()
+
+
+@pytest.mark.parametrize("grid", [(48, 65, 48), (16, 17, 16), (20, 33, 18), (16, 17, 18), (20, 9, 16)])
+def test_nonlin_noalloc_runs_the_same_kernels(grid):
+    """The same kernels and tables as sgpu_nonlin, so the same bits: lengths
+    with two-pass transforms, without them, and one of each."""
+    import torch
+    from simson_b200.bla import Channel, SgpuParams, load_library
+    from simson_b200.fields import channel_field
+
+    nx, ny, nz = grid
+    xl, zl, re, dt = 4 * np.pi, 2 * np.pi, 4200.0, 0.01
+    ch = Channel(nx, ny, nz, re, xl, zl, dt)
+    try:
+        ch.set_velocity(*channel_field(nx, ny, nz, xl, zl, 0.05, 22))
+        ch.prhs()
+        fields = ch.state(5)
+        dev_in = torch.from_numpy(np.ascontiguousarray(np.stack([f.transpose(1, 0, 2) for f in fields]))).cuda()
+        out = torch.zeros((3, ny, nz, nx // 2), dtype=torch.complex128, device="cuda")
+        ch.nonlinbl()
+        h_ref = [ch.get_slot(k) for k in (1, 2, 3)]
+        cfl_ref = ch.scalars()["cfl"]
+    finally:
+        ch.close()
+    lib = load_library()
+    lib.sgpu_nonlin_noalloc.argtypes = [ctypes.POINTER(SgpuParams), ctypes.c_void_p, ctypes.c_void_p,
+                                        ctypes.POINTER(ctypes.c_double), ctypes.c_void_p]
+    prm = SgpuParams(nx, ny, nz, re, xl, zl, dt, 3, 1, 4.0 / 3.0, -2.0 / re, 0.0, 3, 0, 0)
+    cfl = ctypes.c_double(-1.0)
+    rc = lib.sgpu_nonlin_noalloc(ctypes.byref(prm), ctypes.c_void_p(dev_in.data_ptr()),
+                                 ctypes.c_void_p(out.data_ptr()), ctypes.byref(cfl), None)
+    torch.cuda.synchronize()
+    assert rc == 0, rc
+    keep = np.arange(nz) != nz // 2  # no reader takes the oddball plane
+    for a, b in zip(out.cpu().numpy(), h_ref):
+        np.testing.assert_array_equal(a.transpose(1, 0, 2)[keep], b[keep])
+    assert abs(cfl.value * np.pi * dt - cfl_ref) <= 1e-15 * cfl_ref
