@@ -27,8 +27,9 @@ constexpr int LES_TP = 16, LES_KC = 16;
 SB_HD __forceinline__ int les_hpf_ld(int n) { return (n + 7) / 8 * 8; }  // row length of the matrix, k-major
 inline int les_hpf_threads(int n) { return ((n + 7) / 8 * (LES_TP / 2) + 31) / 32 * 32; }
 inline int les_hpf_smem(int n) { return n * LES_TP * 16 + 2 * LES_KC * les_hpf_ld(n) * 8; }
-// whether the tile fits (ny up to about 800; the serial kernel serves the rest)
-inline bool les_hpf_fits(int n) { return les_hpf_smem(n) <= 227 * 1024 && les_hpf_threads(n) <= 1024; }
+// whether the tile fits: ny up to 451 (512 bytes a row); the column solves
+// serve the rest
+inline bool les_hpf_fits(int n) { return les_hpf_smem(n) <= 227 * 1024; }
 
 // Per-row coefficients, LES_ROW doubles per row:
 //   [0..4]  right-hand-side stencil of the high pass (g2 - g1)

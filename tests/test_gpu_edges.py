@@ -7,7 +7,9 @@ that file's tolerances (four times the distance seen, per kind and precision):
   transforms take, in x, in z and in both;
 * Smagorinsky stress: the shortest two-pass lengths, and lengths of the
   general transforms beside two-pass ones;
-* ADM-RT: ny at the ends of the filter product's row tiles and beyond them."""
+* ADM-RT: ny at the ends of the filter product's row tiles, the last ny whose
+  product fits a CTA's shared memory and the next one, which the column solves
+  filter."""
 import importlib.util
 import math
 import os
@@ -65,3 +67,36 @@ def test_smagorinsky(cases, grid):
                                   (16, 161, 16)])
 def test_filter(cases, grid):
     check(cases, "les", "admrt", grid, "fp64", 2)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("ny", [161, 451, 481])
+def test_filtered_velocity(cases, ny, precision):
+    """The filtered velocities themselves, of columns rough enough that the high
+    pass keeps them: 1e-12, the gate of the model's other tests, of six solves
+    of diagonally dominant rows and a sum of ny products."""
+    import numpy as np
+    import torch
+    from simson_b200.bla import Channel
+    nx, nz = 16, 16
+    rng = np.random.default_rng(7)
+    vel = rng.standard_normal((3, nz, ny, nx // 2)) + 1j * rng.standard_normal((3, nz, ny, nx // 2))
+    vel[:, nz // 2] = 0.0
+    vel[:, 0, :, 0] = vel[:, 0, :, 0].real
+    ch = Channel(nx, ny, nz, 4200.0, 4 * math.pi, 2 * math.pi, 0.004, precision=precision)
+    try:
+        ch.set_les(iles=1)
+        ch.set_velocity(*vel)
+        ch.start()
+        got = ch.les_gu()
+    finally:
+        ch.close()
+    if precision == "mixed":  # the stored state is what is filtered
+        vel = vel.real.astype(np.float32).astype(np.float64) + 1j * vel.imag.astype(np.float32).astype(np.float64)
+    filt = cases._Exact(dict(nx=nx, ny=ny, nz=nz, xl=4 * math.pi, zl=2 * math.pi)).high_pass()
+    keep = np.arange(nz) != nz // 2
+    for g, v in zip(got, vel):
+        want = filt(torch.tensor(v.transpose(1, 0, 2)).to(cases._device())).cpu().numpy().transpose(1, 0, 2)
+        err = np.linalg.norm(g[keep] - want[keep]) / np.linalg.norm(want[keep])
+        print(ny, precision, "%.1e" % err)
+        assert err <= 1e-12
