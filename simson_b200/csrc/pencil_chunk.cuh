@@ -34,7 +34,8 @@
 // walks, a third in global and spill loads; FP64 pipe 15 %, DRAM 16 %.  Per
 // launch, before (the better of one thread and one warp per pencil) and now:
 // 48x65x48 60 -> 12 us, 64x97x64 62 -> 23, 192x129x160 591 -> 178,
-// 384x193x384 1810 -> 1250.
+// 384x193x384 1810 -> 1250, 64x257x64 1140 -> 67, 192x257x160 1320 -> 375,
+// 384x257x288 1930 -> 1240.
 #pragma once
 #include "press.cuh"
 #include "step3.cuh"
@@ -49,11 +50,16 @@ constexpr int PC_AREA = 38;                  // exchange area, doubles per threa
 constexpr int PC_WB = 4;                     // chunks a walk reads ahead of its chain
 // rows per chunk: even, so that a row's class is its parity everywhere
 constexpr int PC_MAX_R = 10;
-// resident CTAs per SM the register budget is sized for: four (128
-// registers) of the shortest chunks, so that the 512 CTAs of 64x97x64 are
-// resident at once (0.028 -> 0.021 ms), three (168 registers) of the others,
-// which spill at four (192x129x160 0.16 -> 0.18 ms)
-constexpr int pc_minb(int r) { return r == 4 ? 4 : 3; }
+// Resident CTAs per SM the register budget of k_pencil_c is sized for.  R = 4:
+// four (128 registers, no spills), so that the 512 CTAs of 64x97x64 are
+// resident at once (0.028 -> 0.021 ms).  R = 6, 8: three (168 registers, 20 and
+// 32 bytes spilled); at four they spill more (192x129x160 0.16 -> 0.18 ms).
+// R = 10: two, all that its 79 KB of shared memory a CTA leave room for; held
+// to 168 registers all the same it spilled 328 bytes (384x257x288 1.46 -> 1.24
+// ms, 192x257x160 0.44 -> 0.38, 64x257x64 0.077 -> 0.067).
+constexpr int pc_minb(int r) { return r == 4 ? 4 : r == 10 ? 2 : 3; }
+// the same of k_press_c, which spills nowhere
+constexpr int pc_press_minb(int r) { return r == 4 ? 4 : 3; }
 
 // c'_j of (D^2 - lam) for every stored kx and 0 <= |kz| <= nz/2: out[j][pa],
 // pa = |kz| nx2 + kx; lam = k^2 + shift.  One thread per column and parity.
@@ -109,7 +115,8 @@ __device__ __forceinline__ void pc_copy8(double* dst, const double* src, bool in
 __device__ __forceinline__ void pc_copy_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // Element of a field at a byte offset below 4 GB (one offset register serves
-// every field of a row).
+// every field of a row): a context holds about fifty complex fields, so one of
+// 4 GB does not fit a GPU of 180 GB.
 template <class T>
 __device__ __forceinline__ T& pc_at(void* base, unsigned off) {
   return *reinterpret_cast<T*>(reinterpret_cast<char*>(base) + off);
@@ -891,7 +898,7 @@ __global__ void __launch_bounds__((PC_NT + 31) / 32 * 32, pc_minb(R))
 // 0.58 ms at 192x129x160 for 0.25 GB, one wave of serial walks; this one
 // 0.095.
 template <int R, class VT>
-__global__ void __launch_bounds__((PC_NT + 31) / 32 * 32, pc_minb(R))
+__global__ void __launch_bounds__((PC_NT + 31) / 32 * 32, pc_press_minb(R))
     k_press_c(PressArgs P, const VT* __restrict__ V, Dims g, const double* __restrict__ CV,
               const double2* __restrict__ rows, int G) {
   extern __shared__ __align__(16) unsigned char pc_smem[];
@@ -1027,9 +1034,6 @@ __global__ void __launch_bounds__((PC_NT + 31) / 32 * 32, pc_minb(R))
 
 // Rows per chunk for ny: 0 when ny is beyond the kernel's range
 inline int pencil_chunk_rows(int ny) {
-#ifdef SB_PC_R
-  if ((ny + SB_PC_R - 1) / SB_PC_R <= PC_MAXG) return SB_PC_R;
-#endif
   for (int r = 4; r <= PC_MAX_R; r += 2)
     if ((ny + r - 1) / r <= PC_MAXG) return r;
   return 0;

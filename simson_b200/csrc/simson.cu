@@ -210,22 +210,25 @@ struct sgpu_ctx {
 };
 
 // Whether a group of threads can solve a pencil of this context.  FP64: the
-// chunked kernel.  Mixed: one warp per pencil; the chunked kernel would serve
-// its FP32 storage as well (64x97x64 0.021 against 0.062 ms), but joins its
-// sums in another order, and the mixed path's forcing, rounded to FP32, turns
-// a last-bit difference into its whole rounding noise (4e-6 of p_v, single
-// values up to 7e-4 of its rms), beyond what a change of kernel may show.
+// chunked kernel.  Mixed: one warp per pencil.  The chunked kernel would serve
+// FP32 storage as well (64x97x64 0.021 against 0.062 ms), but joins its sums in
+// another order, and rounding the state to FP32 turns that last bit into the
+// rounding noise of the mixed path: 4e-6 of p_v, single values up to 7e-4 of
+// its rms, where the state is 1e-6 from the solution at 64 bits.  Whether its
+// distance from that solution is no larger, over fields and grids, has not
+// been measured.
 static bool pencil_chunked(const sgpu_ctx* c) { return !c->mixed && pencil_chunk_fits(c->g.nyp); }
 static bool pencil_group_fits(const sgpu_ctx* c) {
   return c->mixed ? pencil_warp_rows(c->g.nyp) > 0 : pencil_chunk_fits(c->g.nyp) != 0;
 }
 // The automatic choice of step 3's pencil kernel.  FP64: the chunked kernel
-// (against one thread per pencil: 48x65x48 0.012 / 0.24 ms, 192x129x160 0.18 /
-// 0.59, 384x193x384 1.25 / 1.81).  Mixed: a warp per pencil up to 8192 pencils
-// (0.062 against 0.29 ms at 64x97x64, 2 048 pencils; 0.28 against 0.58 at
-// 96x129x96, 4 608), one thread per pencil above (0.43 against 0.85 at
-// 192x129x160, 15 360; 1.0 against 5.2 at 384x193x384, 73 728, where it
-// streams near the DRAM bandwidth).
+// for every ny it takes (against one thread per pencil: 48x65x48 0.012 / 0.24
+// ms, 192x129x160 0.18 / 0.59, 384x193x384 1.25 / 1.81, and at the longest
+// chunks 64x257x64 0.067 / 1.14, 256x241x256 0.73 / 1.46, 384x257x288 1.24 /
+// 1.93).  Mixed: a warp per pencil up to 8192 pencils (0.062 against 0.29 ms at
+// 64x97x64, 2 048 pencils; 0.28 against 0.58 at 96x129x96, 4 608), one thread
+// per pencil above (0.43 against 0.85 at 192x129x160, 15 360; 1.0 against 5.2
+// at 384x193x384, 73 728, where it streams near the DRAM bandwidth).
 static bool pencil_group_auto(const sgpu_ctx* c) {
   return pencil_group_fits(c) && (!c->mixed || c->g.NP <= 8192);
 }
