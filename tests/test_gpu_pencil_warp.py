@@ -1,16 +1,18 @@
-"""Step 3 with one warp per pencil (pencil_warp.cuh, sgpu_set_pencil_kernel)
-against the thread-per-pencil kernel that follows the reference's
-elimination order, and against the reference itself.
+"""Step 3 with a group of threads per pencil (sgpu_set_pencil_kernel) against
+the thread-per-pencil kernel that follows the reference's elimination order,
+and against the reference itself.  The group is the chunked kernel in FP64
+(pencil_chunk.cuh) and one warp per pencil in mixed precision
+(pencil_warp.cuh).
 
-Both kernels solve the same tau systems; the warp kernel sums in another
-order (partition method with a cyclic reduction over the lanes, derivatives
-as scans), so results agree to round-off: 5e-11 relative L2 per slot in
-FP64 after a step (the stiff lam solve amplifies round-off: the reference
-built with fused multiply-add differs from itself by 9e-12 on omega_z at
-16x17x16 after two steps; the warp kernel is at 1.2e-11 there), 1e-5 under
-SGPU_MIXED (whose u, v, w, omega are stored in FP32 -- one rounding step is
-6e-8 -- and whose gate against FP64 is 1e-5).  The FP64 warp kernel also meets the
-config-A gate against the reference (u, v, w within 1e-11 after ten steps)."""
+All solve the same tau systems and sum in another order (chunk recurrences, or
+the partition method with a cyclic reduction over the lanes; derivatives as
+scans), so results agree to round-off: 5e-11 relative L2 per slot in FP64 after
+a step (the stiff lam solve amplifies round-off: the reference built with fused
+multiply-add differs from itself by 9e-12 on omega_z at 16x17x16 after two
+steps; the chunked kernel is at 2e-12 and below), 1e-5 under SGPU_MIXED (whose
+u, v, w, omega are stored in FP32 -- one rounding step is 6e-8 -- and whose gate
+against FP64 is 1e-5).  Where the reference is there to run, the FP64 kernel
+also meets its config-A gate (u, v, w within 1e-11 after ten steps)."""
 import numpy as np
 import pytest
 
