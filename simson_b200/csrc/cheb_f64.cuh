@@ -86,7 +86,8 @@ __global__ void __launch_bounds__(Chb2<L>::threads, f2_minb(Chb2<L>::threads))
   }
 }
 
-// L = 2 (ny - 1) of the y resolutions that runs use
+// L = 2 (ny - 1): ny = 9 and 17 to 241, ny - 1 of factors 2, 3, 5, but for ny =
+// 11, 13 and 251, which split too and take k_cheb; 512 (ny = 257) has no split
 #define SB_CHB2_LENGTHS(X)                                                                                       \
   X(16) X(32) X(36) X(40) X(48) X(60) X(64) X(72) X(80) X(96) X(100) X(108) X(120) X(128) X(144) X(160) X(180)    \
   X(192) X(200) X(216) X(240) X(256) X(288) X(300) X(320) X(324) X(360) X(384) X(400) X(432) X(480)

@@ -481,10 +481,11 @@ constexpr int cplan_max_nb(int n) {
 // indices and the twiddle powers once for both and its accesses are 16 bytes;
 // the values are the same.  Measured in the x pass: n = 288 (192x129x160) 0.193
 // -> 0.160 ms, the step 3.58 -> 3.40.  Not for short lengths, whose CTAs have
-// too few threads then (n = 96: 34 -> 35 us; n = 150: 48 -> 41, but steps of
-// several contexts at once 2.69 -> 2.80 ms), and not for the longest, where
-// four CTAs fill the shared memory and leave other contexts' kernels no place
-// beside them (n = 576: alone 1.01 -> 0.89 ms, three contexts' steps 21.3 -> 21.9).
+// too few threads then (n = 96: 34 -> 35 us).  n = 150 and 576 are a choice for
+// several contexts at work at once, whose steps got slower (2.69 -> 2.80 ms,
+// 21.3 -> 21.9: at 576 four CTAs fill the shared memory and leave the others'
+// kernels no place beside them); a lone context gives up 48 -> 41 us and 1.01
+// -> 0.89 ms of an x pass for it.  Of the lengths between only 288 was measured.
 // Not in cfft_io either: two columns from and to global memory made the z
 // inverse's accesses 16-byte pieces of a row, 0.51 -> 0.84 ms.
 template <class T, int B, int N>

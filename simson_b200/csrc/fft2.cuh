@@ -274,8 +274,11 @@ constexpr int f2_threads(int items) { return (items + 31) / 32 * 32; }
 // registers
 constexpr int f2_minb(int threads) { return 12 * 32 / threads > 0 ? 12 * 32 / threads : 1; }
 
-// Lengths with two-pass kernels: the 3/2-padded lengths of grid sizes 16 to
-// 384 with factors 2, 3, 5 that runs use.
+// Lengths with two-pass kernels: 3/2 of 27 grid sizes from 16 to 384.  Every
+// length is five kernels to build, so not all that split are here: 27, 30, 45,
+// 54, 75, 81, 162 and 375 (grid sizes 18, 20, 30, 36, 50, 54, 108, 250) split
+// too and take the runtime plan.  243, 405, 486 and 540 have no split with both
+// sides within F2_MAX_R.
 #define SB_F2_LENGTHS_A(X) X(24) X(36) X(48) X(60) X(72) X(90) X(96) X(108) X(120)
 #define SB_F2_LENGTHS_B(X) X(135) X(144) X(150) X(180) X(192) X(216) X(225)
 #define SB_F2_LENGTHS_C(X) X(240) X(270) X(288) X(300) X(324) X(360)

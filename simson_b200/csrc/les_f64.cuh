@@ -334,7 +334,10 @@ __global__ void __launch_bounds__(LF_XT) k_sgs_tau_x2(SgsBufs B, SgsGrid G, cons
   lf_xfwd<N, C, C, 6>(B.tauz6 + row, fs, G.nx2, E, tw, t, LF_XT);
 }
 
-// lengths of LES grids (nx and nz multiples of four)
+// Lengths nx, nz up to 128, the coarse grids that these models are for (and
+// multiples of four, as the models ask).  20 and the 14 lengths of factors 2, 3,
+// 5 from 144 to 384 split too; they take the kernels of les_dyn.cuh, each
+// length being eight more kernels to build.
 #define SB_LF_LENGTHS(X) X(16) X(24) X(32) X(36) X(40) X(48) X(60) X(64) X(72) X(80) X(96) X(100) X(108) X(120) X(128)
 
 }  // namespace sb

@@ -174,7 +174,9 @@ __global__ void __launch_bounds__(XYS_MT) k_xys_moments(const double* __restrict
   for (int k = 0; k < NACC; ++k) part[((size_t)grp * XYS_NACC_P + k) * plane + (size_t)y * G.nx + j] = acc[k];
 }
 
-// lengths nx, nz of grids whose statistics are taken
+// Lengths nx, nz: the multiples of four from 32 to 384 of factors 2, 3, 5.  The
+// others with a split (16 to 30, 50, 54, 90, 150, 162, 250, 270) take xys.cuh's
+// kernels, each length being four more to build.
 #define SB_XYS_LENGTHS(X)                                                                                           \
   X(32) X(36) X(40) X(48) X(60) X(64) X(72) X(80) X(96) X(100) X(108) X(120) X(128) X(144) X(160) X(180) X(192)      \
   X(200) X(216) X(240) X(256) X(288) X(300) X(320) X(324) X(360) X(384)
