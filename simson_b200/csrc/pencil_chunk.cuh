@@ -29,9 +29,10 @@
 // sums of the same walk.  A Chebyshev derivative pair (D, D^2) is one walk of
 // chunk sums.
 //
-// What bounds it (ncu at 192x193x96, R = 8): the latency of a CTA, about 60 000
-// cycles at 12 warps per SM, a third of them at the barriers around the
-// walks, a third in global and spill loads; FP64 pipe 15 %, DRAM 16 %.  Per
+// What bounds it (ncu at 192x129x160, R = 6): the latency of a CTA at 12 warps
+// per SM.  It issues 19 % of the time; the barriers around the walks, in which
+// one warp of four works, come first among the stalls (3.4 per issue), its
+// loads second (2.6); FP64 pipe 14 %, DRAM 25 %.  Per
 // launch, before (the better of one thread and one warp per pencil) and now:
 // 48x65x48 60 -> 12 us, 64x97x64 62 -> 23, 192x129x160 591 -> 178,
 // 384x193x384 1810 -> 1250, 64x257x64 1140 -> 67, 192x257x160 1320 -> 375,
