@@ -1170,6 +1170,7 @@ static int enqueue_linear(sgpu_ctx* c) {
       ts = c->tau_next;
       c->tau_next = (c->tau_next + 1) % c->prm.nst;
       c->tau_key[ts] = anbn;
+      c->step_valid = false;  // a captured step finds the stages by place
       prof_mark(c, K_OTHER);
       pencil_tau_coef(c->stream, c->tau_l + ts * col, g, c->alfa, c->beta, 2.0 * P.re / anbn);
       c->launches++;
@@ -1190,6 +1191,7 @@ static int enqueue_linear(sgpu_ctx* c) {
     hs = c->hom_next;
     c->hom_next = (c->hom_next + 1) % c->prm.nst;
     c->hom_key[hs] = anbn;
+    c->step_valid = false;  // a captured step finds the stages by place
     prof_mark(c, K_OTHER);
     if (c->mixed)
       mixed_pencil_hom(c->stream, B, g, c->alfa, c->beta, P.re, anbn, c->hom_vh + hs * fld,
