@@ -24,7 +24,9 @@
 // which the boundary row (the sum over the class) fixes.  Then
 //   x_j = P_j + PM_j X + N_j Y.
 // |c'| and |c' rho| are below 1 (diagonally dominant rows), so every response
-// decays.  phi_h (zero forcing, wall values 1) is Yq N / sum Q of the same
+// decays -- but at the two truncated last rows, whose c' = -lam / (4 m (m + 1)), m
+// = j - 1, passes 1 at large lam: they feed no row but the boundary's, and the
+// reference's order has them so too.  phi_h (zero forcing, wall values 1) is Yq N / sum Q of the same
 // walk; v_h is a third column of the v solve, and the wall slopes of v are
 // sums of the same walk.  A Chebyshev derivative pair (D, D^2) is one walk of
 // chunk sums.
