@@ -19,17 +19,18 @@
 // truncated last rows): two first-order recurrences per parity class without
 // a division.  A chunk solves them with zero inflow (P), keeps its response
 // PM to the two rows above it and N to the two rows below it, and one warp
-// per parity walks the chunk summaries: down for the inflow X from above, up
-// for the inflow Y from below as Yp + y Yq with the class's first unknown y,
-// which the boundary row (the sum over the class) fixes.  Then
+// walks the chunk summaries, a lane per parity, column and pencil: down for the
+// inflow X from above, up for the inflow Y from below as Yp + y Yq with the
+// class's first unknown y, which the boundary row (the sum over the class)
+// fixes.  Then
 //   x_j = P_j + PM_j X + N_j Y.
 // |c'| and |c' rho| are below 1 (diagonally dominant rows), so every response
-// decays -- but at the two truncated last rows, whose c' = -lam / (4 m (m + 1)), m
-// = j - 1, passes 1 at large lam: they feed no row but the boundary's, and the
-// reference's order has them so too.  phi_h (zero forcing, wall values 1) is Yq N / sum Q of the same
-// walk; v_h is a third column of the v solve, and the wall slopes of v are
-// sums of the same walk.  A Chebyshev derivative pair (D, D^2) is one walk of
-// chunk sums.
+// decays -- but at the two truncated last rows, whose c' = -lam / (4 m (m + 1)),
+// m = j - 1, passes 1 at large lam: they feed no row but the boundary's, and
+// the reference's order has them so too.  phi_h (zero forcing, wall values 1)
+// is Yq N / sum Q of the same walk; v_h is a third column of the v solve, and
+// the wall slopes of v are sums of the same walk.  A Chebyshev derivative pair
+// (D, D^2) is one walk of chunk sums.
 //
 // What bounds it (ncu at 192x129x160, R = 6): the latency of a CTA at 12 warps
 // per SM.  It issues 19 % of the time; the barriers around the walks, in which
