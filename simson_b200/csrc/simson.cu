@@ -285,6 +285,7 @@ static int make_tw(Tw& t, int n) {
   CK(cudaMalloc(&t.f, n * sizeof(float2)));
   CK(cudaMemcpy(t.d, hd.data(), n * sizeof(double2), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(t.f, hf.data(), n * sizeof(float2), cudaMemcpyHostToDevice));
+  CK(cudaStreamSynchronize(cudaStreamLegacy));  // the context's stream does not wait for this one
   return SGPU_OK;
 }
 
@@ -540,7 +541,11 @@ extern "C" int sgpu_init(const sgpu_params* prm, sgpu_ctx** out) {
   const char* pw = getenv("SIMSON_PENCIL_WARP");
   c->pencil_group = pw ? (pw[0] == '1' && pencil_group_fits(c)) : pencil_group_auto(c);
   if ((rc = pencil_bufs(c, c->pencil_group))) return fail(rc);
-  if (cudaDeviceSynchronize() != cudaSuccess) return fail(SGPU_E_CUDA);
+  // the copies above went over the legacy stream, which the context's does not
+  // wait for; a synchronisation of the device would break a step that another
+  // thread's context is capturing
+  if (cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess || cudaStreamSynchronize(c->stream) != cudaSuccess)
+    return fail(SGPU_E_CUDA);
   *out = c;
   return SGPU_OK;
 }

@@ -65,3 +65,44 @@ def test_smaller_context_leaves_the_larger_one(grid, precision, what, les):
         ch.close()
     for a, b in zip(alone, got):
         np.testing.assert_array_equal(a, b)
+
+
+def test_contexts_in_several_threads():
+    """Contexts made, stepped (with captured steps), sampled and closed by
+    several host threads at once give what they give one after another."""
+    import threading
+    from simson_b200.bla import FP64, MIXED, Channel
+    runs = [((16, 161, 16), FP64, dict(iles=1)), ((16, 33, 16), FP64, dict(iles=1)), ((16, 193, 16), MIXED, None),
+            ((144, 17, 16), FP64, dict(iles=2)), ((200, 17, 50), MIXED, None), ((48, 65, 48), FP64, None)]
+    xl, zl = 4 * np.pi, 2 * np.pi
+    fields = [channel_field(*grid, xl, zl, 0.05, 5) for grid, _, _ in runs]
+
+    def work(i, out):
+        grid, precision, les = runs[i]
+        for _ in range(3):
+            ch = Channel(*grid, 4200.0, xl, zl, 0.002, precision=precision)
+            try:
+                if les:
+                    ch.set_les(**les)
+                ch.set_velocity(*fields[i])
+                ch.start()
+                ch.step(3)
+                ch.xys_sample()
+                out[i].append(ch.state(7) + [ch.xys()[0], ch.pressure()])
+            finally:
+                ch.close()
+
+    alone = [[] for _ in runs]
+    for i in range(len(runs)):
+        work(i, alone)
+    at_once = [[] for _ in runs]
+    threads = [threading.Thread(target=work, args=(i, at_once)) for i in range(len(runs))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for a, b in zip(alone, at_once):
+        assert len(b) == 3
+        for r in b:
+            for p, q in zip(a[0], r):
+                np.testing.assert_array_equal(p, q)
